@@ -66,8 +66,9 @@ typedef struct { float x, y, u, v, sn; } opiv_vector;
 
 /* peak code per window: py * W + px of the first peak in the quadrant-
  * swapped plane (zero lag at (W/2, W/2)), or -1 when fewer than two peaks;
- * OPIV_PEAK_EXACT is or-ed in when the window was decided by the exact
- * double-precision pass rather than the FP32 pass. */
+ * OPIV_PEAK_EXACT is or-ed in when the window was decided by the exact pass
+ * (exact correlation sums, or the reference's double arithmetic where those
+ * leave a tie) rather than the FP32 pass. */
 #define OPIV_PEAK_EXACT 0x40000000
 #define OPIV_PEAK_MASK 0x0000FFFF
 

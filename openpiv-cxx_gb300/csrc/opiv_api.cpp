@@ -114,6 +114,19 @@ std::vector<double2> reference_twiddles(uint32_t n, int dir)
 int exact_blocks(int device) { return 2 * device_sm_count(device); }
 int exact_all_blocks(int device) { return 8 * device_sm_count(device); }
 
+// Flagged windows whose planes a pass keeps for refine_window: particle
+// images flag up to one window in a hundred; beyond this room (or 4 MiB)
+// the exact kernel decides them from the frames alone.
+int32_t flag_capacity(int64_t n_win, uint32_t ia)
+{
+    const int64_t room = (int64_t)(4u << 20) / (int64_t)(sizeof(float) * flag_record_floats((int)ia));
+    return (int32_t)std::min({ n_win, 64 + n_win / 32, room });
+}
+size_t flag_plane_bytes(int32_t cap, uint32_t ia)
+{
+    return sizeof(float) * flag_record_floats((int)ia) * (size_t)cap;
+}
+
 bool is_tc(int precision)
 {
     return precision == OPIV_PREC_TC_SPLIT_BF16 || precision == OPIV_PREC_TC_BF16 ||
@@ -174,6 +187,8 @@ struct opiv_plan {
     int32_t* d_peak = nullptr;
     unsigned int* d_flag_count = nullptr;
     int32_t* d_flag_list = nullptr;
+    float* d_flag_planes = nullptr;     // planes of the first flag_cap flagged windows
+    int32_t flag_cap = 0;
     double2* d_tw = nullptr;            // forward then reverse, ia entries each
     unsigned int* h_flag_count = nullptr;   // pinned copy of the last count
     bool timing = false;
@@ -195,6 +210,7 @@ struct opiv_plan {
     cudaStream_t cs2 = nullptr;                 // compute stream of odd pairs
     unsigned int* p_flag_count[kPipeSlots] = {};
     int32_t* p_flag_list[kPipeSlots] = {};
+    float* p_flag_planes[kPipeSlots] = {};
     void* p_fa[kPipeSlots] = {};
     void* p_fb[kPipeSlots] = {};
     opiv_vector* p_vec[kPipeSlots] = {};
@@ -226,6 +242,7 @@ void plan_free(opiv_plan* p)
     cudaFree(p->d_peak);
     cudaFree(p->d_flag_count);
     cudaFree(p->d_flag_list);
+    cudaFree(p->d_flag_planes);
     cudaFree(p->d_tw);
     cudaFree(p->d_disp);
     cudaFree(p->d_tc);
@@ -245,6 +262,7 @@ void plan_free(opiv_plan* p)
     for (int k = 0; k < opiv_plan::kPipeSlots; ++k) {
         cudaFree(p->p_flag_count[k]);
         cudaFree(p->p_flag_list[k]);
+        cudaFree(p->p_flag_planes[k]);
     }
     if (p->up) cudaStreamDestroy(p->up);
     if (p->down) cudaStreamDestroy(p->down);
@@ -271,6 +289,8 @@ PivParams base_params(const opiv_plan* p)
     k.kappa = kKappa;
     k.flag_count = p->d_flag_count;
     k.flag_list = p->d_flag_list;
+    k.flag_planes = p->d_flag_planes;
+    k.flag_cap = p->flag_cap;
     k.tw_fwd = p->d_tw;
     k.tw_rev = p->d_tw + p->ia;
     return k;
@@ -279,8 +299,8 @@ PivParams base_params(const opiv_plan* p)
 // One pass: FP32 kernel over all windows, then the exact pass over the
 // flagged ones.  Two kernel launches.  `prev` (may be null): the previous
 // pass of a multi-pass chain, whose integer displacements offset frame B.
-// flag_count / flag_list: the exact pass's scratch (null: the plan's own;
-// passes that may run concurrently need their own).
+// flag_count / flag_list / flag_planes: the exact pass's scratch (null: the
+// plan's own; passes that may run concurrently need their own).
 // The parameters of one pass of plan p over frames fa, fb; `prev`: the
 // previous pass of a multi-pass chain (window offsetting) or null.
 PivParams pass_params(const opiv_plan* p, const void* fa, const void* fb, size_t pitch,
@@ -308,12 +328,14 @@ PivParams pass_params(const opiv_plan* p, const void* fa, const void* fb, size_t
 
 int run_pass(opiv_plan* p, const void* fa, const void* fb, size_t pitch, opiv_vector* vec,
              int32_t* peak, cudaStream_t s, const opiv_plan* prev = nullptr,
-             unsigned int* flag_count = nullptr, int32_t* flag_list = nullptr)
+             unsigned int* flag_count = nullptr, int32_t* flag_list = nullptr,
+             float* flag_planes = nullptr)
 {
     PivParams k = pass_params(p, fa, fb, pitch, vec, peak, prev);
     if (flag_count) {
         k.flag_count = flag_count;
         k.flag_list = flag_list;
+        k.flag_planes = flag_planes;
     }
     CUDA_TRY(cudaMemsetAsync(k.flag_count, 0, sizeof(unsigned int), s));
     if (is_tc(p->precision)) {
@@ -488,6 +510,11 @@ int plan_create(opiv_plan** out, uint32_t img_w, uint32_t img_h, int dtype, uint
         return done(cuda_fail(e, "cudaMalloc(flag count)"));
     if ((e = cudaMalloc(&p->d_flag_list, sizeof(int32_t) * p->n_win)) != cudaSuccess)
         return done(cuda_fail(e, "cudaMalloc(flag list)"));
+    if (!tc_only) {   // passes of the tensor-core path flag nothing
+        p->flag_cap = flag_capacity(p->n_win, ia);
+        if ((e = cudaMalloc(&p->d_flag_planes, flag_plane_bytes(p->flag_cap, ia))) != cudaSuccess)
+            return done(cuda_fail(e, "cudaMalloc(flagged planes)"));
+    }
     if ((e = cudaMemset(p->d_flag_count, 0, sizeof(unsigned int))) != cudaSuccess)
         return done(cuda_fail(e, "cudaMemset"));
     if ((e = cudaMallocHost(&p->h_flag_count, sizeof(unsigned int))) != cudaSuccess)
@@ -642,7 +669,9 @@ int opiv_process_pairs(opiv_plan* plan, int64_t n_pairs, const void* const* fram
             if ((e = cudaEventCreateWithFlags(&plan->ev_done[k], cudaEventDisableTiming)) != cudaSuccess) break;
             if ((e = cudaEventCreateWithFlags(&plan->ev_down[k], cudaEventDisableTiming)) != cudaSuccess) break;
             if ((e = cudaMalloc(&plan->p_flag_count[k], sizeof(unsigned int))) != cudaSuccess) break;
-            e = cudaMalloc(&plan->p_flag_list[k], sizeof(int32_t) * plan->n_win);
+            if ((e = cudaMalloc(&plan->p_flag_list[k], sizeof(int32_t) * plan->n_win)) != cudaSuccess) break;
+            if (plan->flag_cap > 0)
+                e = cudaMalloc(&plan->p_flag_planes[k], flag_plane_bytes(plan->flag_cap, plan->ia));
         }
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&plan->up, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&plan->down, cudaStreamNonBlocking);
@@ -679,7 +708,7 @@ int opiv_process_pairs(opiv_plan* plan, int64_t n_pairs, const void* const* fram
         if (i >= S) CUDA_TRY(cudaStreamWaitEvent(cs, plan->ev_down[k], 0));
         const int rc = run_pass(plan, plan->p_fa[k], plan->p_fb[k], row, plan->p_vec[k],
                                 out_peak ? plan->p_peak[k] : nullptr, cs, nullptr,
-                                plan->p_flag_count[k], plan->p_flag_list[k]);
+                                plan->p_flag_count[k], plan->p_flag_list[k], plan->p_flag_planes[k]);
         if (rc != OPIV_OK) return done(rc);
         CUDA_TRY(cudaEventRecord(plan->ev_done[k], cs));
         CUDA_TRY(cudaStreamWaitEvent(plan->down, plan->ev_done[k], 0));
@@ -849,6 +878,7 @@ struct batch_queue_pass {
     std::vector<PivQueue> groups;       // host copies, passed by value at launch
     unsigned int* d_ctr = nullptr;      // per group: dequeue head, flagged windows
     int32_t* d_flags = nullptr;         // per group: its flag list (combined window numbers)
+    float* d_planes = nullptr;          // per group: planes of its first flagged windows
     PivParams* d_items = nullptr;       // per group: its descriptors (kQueueMaxItems slots)
     uint8_t* d_task_item = nullptr;     // per group: the pair of every task
     int ia = 0, dtype = 0, mode = 0, limit = 0;
@@ -903,6 +933,7 @@ void batch_free_queue(opiv_batch* b)
     for (batch_queue_pass& q : b->qp) {
         cudaFree(q.d_ctr);
         cudaFree(q.d_flags);
+        cudaFree(q.d_planes);
         cudaFree(q.d_items);
         cudaFree(q.d_task_item);
     }
@@ -956,6 +987,7 @@ int batch_queue_setup(opiv_batch* b)
         }
         q.groups.resize(n_groups);
         std::vector<int64_t> flag_off(n_groups + 1, 0);   // each group's flag list in d_flags
+        std::vector<int64_t> plane_off(n_groups + 1, 0);  // each group's records in d_planes
         std::vector<int64_t> task_off(n_groups + 1, 0);   // each group's task pairs in d_task_item
         std::vector<uint8_t> task_item;
         const size_t px = px_bytes(q.dtype);
@@ -989,12 +1021,15 @@ int batch_queue_setup(opiv_batch* b)
             pq.first_task[pq.n_items] = (int)tasks;
             pq.first_win[pq.n_items] = (int)wins;
             flag_off[g + 1] = flag_off[g] + (wins > 0 ? wins : 1);
+            plane_off[g + 1] = plane_off[g] + flag_capacity(wins, q.ia);
             task_off[g + 1] = task_off[g] + tasks;
         }
         if (rc != OPIV_OK) break;
         cudaError_t e;
         if ((e = cudaMalloc(&q.d_ctr, 2 * sizeof(unsigned int) * n_groups)) != cudaSuccess ||
             (e = cudaMalloc(&q.d_flags, sizeof(int32_t) * flag_off[n_groups])) != cudaSuccess ||
+            (e = cudaMalloc(&q.d_planes, flag_plane_bytes((int32_t)std::max<int64_t>(1, plane_off[n_groups]), q.ia))) !=
+                cudaSuccess ||
             (e = cudaMalloc(&q.d_items, sizeof(PivParams) * kQueueMaxItems * n_groups)) != cudaSuccess ||
             (e = cudaMalloc(&q.d_task_item, task_item.size() + 1)) != cudaSuccess) {
             rc = cuda_fail(e, "cudaMalloc(work queue)");
@@ -1008,6 +1043,8 @@ int batch_queue_setup(opiv_batch* b)
             for (int j = 0; j < pq.n_items; ++j) {   // the group's one flag list
                 pq.items[j].flag_count = q.d_ctr + 2 * g + 1;
                 pq.items[j].flag_list = q.d_flags + flag_off[g];
+                pq.items[j].flag_planes = q.d_planes + plane_off[g] * flag_record_floats(q.ia);
+                pq.items[j].flag_cap = (int32_t)(plane_off[g + 1] - plane_off[g]);
             }
             pq.items_g = q.d_items + (size_t)kQueueMaxItems * g;
             pq.task_item = q.d_task_item + task_off[g];

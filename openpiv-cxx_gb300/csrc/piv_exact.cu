@@ -19,13 +19,15 @@
 //     in double.
 //
 // It serves two purposes: it re-decides the windows the FP32 kernel flagged
-// as uncertain, and it is the device FP64 correlation used by the exact
-// per-window API.  One CTA of 256 threads handles one window at a time;
+// as uncertain (after refine_window below, which settles nearly all of them
+// from a few exact sums), and it is the device FP64 correlation used by the
+// exact per-window API.  One CTA of 256 threads handles one window at a time;
 // CTAs stride over the work list.  FP64 is slow on this part, so the hot path only sends
 // the rare flagged windows here.
 
 #include <atomic>
 #include <cstdint>
+#include <type_traits>
 #include <cuda_runtime.h>
 
 #include "offsets.cuh"
@@ -111,9 +113,10 @@ __device__ __forceinline__ void window_origin(const PivParams& p, int64_t w, int
         bx = p.win_xy[2 * w];
         by = p.win_xy[2 * w + 1];
     } else {
-        const int64_t gy = w / p.gnx, gx = w - gy * p.gnx;
-        bx = p.gx0 + (int)gx * p.gdx;
-        by = p.gy0 + (int)gy * p.gdy;
+        // a plan holds at most 2^31 - 1 windows
+        const int gy = (int)((unsigned)w / (unsigned)p.gnx);
+        bx = p.gx0 + ((int)w - gy * p.gnx) * p.gdx;
+        by = p.gy0 + gy * p.gdy;
     }
 }
 
@@ -272,6 +275,263 @@ __device__ __forceinline__ void exact_window(const PivParams& p, const int64_t w
     __syncthreads();
 }
 
+// ---- a flagged window from exact sums -----------------------------------------
+// Nearly every window that the FP32 kernel cannot decide hangs on a handful
+// of plane values: two peaks within its error bound, or a second peak or a
+// fit whose value needs more digits.  Those values are direct correlation
+// sums, sum_p a[p] b[p + lag]: whole numbers for 8/16-bit frames (at most
+// 2^44, kept in 64 bits), FP64 sums for float frames.  So instead of three
+// 2-D transforms in FP64 (about 160,000 FP64 operations for a 32 px window at
+// two per cycle and SM: 40 us for one CTA at best), the CTA takes the FP32
+// plane that the window was flagged with, finds every cell that could be one
+// of the two highest maxima within the FP32 error bound, and evaluates those
+// cells and their neighbours exactly.  In units of W^2 times a plane value,
+// REAL mode's plane (spectrum column 0 and rows 0, W/2 left out) is
+//   V = W^2 R - W (rows + columns + (-1)^dy alternating)
+//         + Sa Sb + (-1)^dy Ta Tb,
+// where rows and columns are the 1-D correlations of the windows' row and
+// column sums, alternating that of the (-1)^y-weighted column sums, S and T
+// the totals of the plain and the weighted sums: whole numbers again.
+// Returns false, with nothing written, where the exact kernel has to decide:
+// ties and signs within the reference's own FP64 rounding, more than
+// kMaxCand candidates, non-finite planes.
+// The launch's time with the FP64 transforms and with this: a 4096 x 4096
+// pass of 32 px windows at step 8 (4 flagged) 111 -> 12 us; 2048 x 1536, 16 px
+// at step 8 (78 flagged) 48 -> 9 us; 2048 x 2048, 64 px at step 16 (2 flagged)
+// 360 -> 20 us; none flagged 3 us.  What is left is a chain of dependent loads,
+// block barriers and FP64 logarithms of one window.
+constexpr int kMaxCand = 16;
+
+struct refine_shared {
+    long long val[5 * kMaxCand];   // or doubles: centre, left, right, up, down
+    float top0[kThreads / 32], top1[kThreads / 32];
+    int key[kMaxCand];
+    int count;
+    int ok;
+};
+
+template <typename T>
+__device__ __forceinline__ T warp_total(T v)
+{
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+template <typename PixT>
+__device__ __forceinline__ bool refine_window(const PivParams& p, const int64_t w, const int W, const int mode,
+                                              const int sy0, const int sy1, const int sx0, const int sx1,
+                                              const float* rec, unsigned char* smem, refine_shared& rs)
+{
+    constexpr bool kFloat = sizeof(PixT) == 4;
+    using Px = typename std::conditional<kFloat, double, uint32_t>::type;
+    using Acc = typename std::conditional<kFloat, double, long long>::type;
+    const int t = threadIdx.x, T = blockDim.x, lane = t & 31, warp = t >> 5, warps = T >> 5;
+    const int N = W * W, m = W - 1, lg = 31 - __clz(W);
+    const float dlt = rec[N];
+    if (!(dlt > 1e-30f && dlt < 1e30f)) return false;   // block-uniform; also blank windows and NaN
+
+    Px* A = reinterpret_cast<Px*>(smem);
+    Px* B = A + N;
+    float* C = reinterpret_cast<float*>(B + N);
+    Acc* prof = reinterpret_cast<Acc*>(C + N);   // REAL: 6 W sums
+    int bx, by, ox, oy;
+    window_origin(p, w, bx, by);
+    b_offset(p, W, bx, by, ox, oy);
+    {
+        const PixT* fa = reinterpret_cast<const PixT*>(p.fa);
+        const PixT* fb = reinterpret_cast<const PixT*>(p.fb);
+        const size_t pitch = p.pitch / sizeof(PixT);
+        for (int i = t; i < N; i += T) {
+            const int y = i >> lg, x = i & m;
+            A[i] = (Px)__ldg(fa + (size_t)(by + y) * pitch + bx + x);
+            B[i] = (Px)__ldg(fb + (size_t)(by + oy + y) * pitch + bx + ox + x);
+            C[i] = rec[i];
+        }
+    }
+    if (t == 0) rs.count = 0;
+    __syncthreads();
+
+    // the two highest cells that are maxima whatever the rounding: nothing
+    // below the second of them (less the bound) matters
+    const float ninf = -__int_as_float(0x7f800000);
+    auto scanned = [&](int k) {
+        const int y = k >> lg, x = k & m;
+        return y >= sy0 && y < sy1 && x >= sx0 && x < sx1;
+    };
+    auto rise = [&](int k) {   // highest neighbour minus the cell
+        return fmaxf(fmaxf(C[k - 1], C[k + 1]), fmaxf(C[k - W], C[k + W])) - C[k];
+    };
+    float s0 = ninf, s1 = ninf;
+    for (int k = t; k < N; k += T) {
+        if (!scanned(k)) continue;
+        const float c = rise(k) < -dlt ? C[k] : ninf;
+        s1 = fmaxf(s1, fminf(s0, c));
+        s0 = fmaxf(s0, c);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        const float q0 = __shfl_xor_sync(0xffffffffu, s0, o), q1 = __shfl_xor_sync(0xffffffffu, s1, o);
+        s1 = fmaxf(fmaxf(s1, q1), fminf(s0, q0));
+        s0 = fmaxf(s0, q0);
+    }
+    if (lane == 0) {
+        rs.top0[warp] = s0;
+        rs.top1[warp] = s1;
+    }
+    if (mode == kModeReal) {
+        // row sums of a and b, column sums, (-1)^y-weighted column sums
+        for (int i = t; i < 4 * W; i += T) {
+            const Px* X = (i & 1) ? B : A;
+            const int l = (i >> 1) & m;
+            Acc s = 0, h = 0;
+            if (i < 2 * W) {
+                for (int x = 0; x < W; ++x) s += (Acc)X[l * W + x];
+                prof[(i & 1) * W + l] = s;
+            } else {
+                for (int y = 0; y < W; ++y) {
+                    const Acc v = (Acc)X[y * W + l];
+                    s += v;
+                    h += (y & 1) ? -v : v;
+                }
+                prof[(2 + (i & 1)) * W + l] = s;
+                prof[(4 + (i & 1)) * W + l] = h;
+            }
+        }
+    }
+    __syncthreads();
+    float g0 = ninf, g1 = ninf;
+    for (int i = 0; i < warps; ++i) {
+        g1 = fmaxf(fmaxf(g1, rs.top1[i]), fminf(g0, rs.top0[i]));
+        g0 = fmaxf(g0, rs.top0[i]);
+    }
+    const float floor_c = g1 - dlt;
+    for (int k = t; k < N; k += T) {
+        if (scanned(k) && C[k] >= floor_c && rise(k) <= dlt) {
+            const int n = atomicAdd(&rs.count, 1);
+            if (n < kMaxCand) rs.key[n] = k;
+        }
+    }
+    __syncthreads();
+    const int n = rs.count;
+    if (n > kMaxCand) {
+        __syncthreads();   // the next window resets the count
+        return false;
+    }
+
+    // exact values, one warp per value
+    Acc* val = reinterpret_cast<Acc*>(rs.val);
+    for (int q = warp; q < 5 * n; q += warps) {
+        const int k = rs.key[q / 5], j = q % 5;
+        const int dx = (k & m) + (j == 2) - (j == 1) - W / 2, dy = (k >> lg) + (j == 4) - (j == 3) - W / 2;
+        Acc s = 0;
+#pragma unroll 8
+        for (int i = lane; i < N; i += 32) {
+            const int y = i >> lg, x = i & m;
+            const Px a = A[i], b = B[(((y + dy) & m) << lg) + ((x + dx) & m)];
+            if constexpr (kFloat) s = fma(a, b, s);
+            else s += (long long)((unsigned long long)a * b);
+        }
+        s *= N;
+        if (mode == kModeReal) {
+            const Acc sg = (dy & 1) ? -1 : 1;
+            Acc c = 0, sa = 0, sb = 0, ta = 0, tb = 0;
+            for (int i = lane; i < W; i += 32) {
+                const int iy = (i + dy) & m, ix = (i + dx) & m;
+                c += prof[i] * prof[W + iy] + prof[2 * W + i] * prof[3 * W + ix] +
+                     sg * prof[4 * W + i] * prof[5 * W + ix];
+                sa += prof[i];
+                sb += prof[W + i];
+                ta += prof[4 * W + i];
+                tb += prof[5 * W + i];
+            }
+            s -= W * c;
+            s = warp_total(s) + warp_total(sa) * warp_total(sb) + sg * warp_total(ta) * warp_total(tb);
+        } else {
+            s = warp_total(s);
+        }
+        if (lane == 0) val[q] = s;
+    }
+    __syncthreads();
+
+    // the decision, by one warp (every lane alike up to the logarithms)
+    if (warp == 0) {
+        // dlt bounds the FP32 plane's rounding, in units of 4 W^2; the
+        // reference's FP64 transforms round 2^29 times finer.  32 times that,
+        // in units of W^2, also covers the sums here (two neighbouring whole
+        // numbers are W^2 apart)
+        const double eps = (double)dlt * 1.4901161193847656e-8;
+        const Acc tol = kFloat ? (Acc)eps : (Acc)eps + 1;
+        bool ok = true;
+        int k0 = -1, found = 0;
+        Acc v0 = 0, v1 = 0;
+        for (int i = 0; i < n; ++i) {
+            const Acc* v = val + 5 * i;
+            const Acc c = v[0];
+            bool peak = true, below = false;
+            for (int j = 1; j < 5; ++j) {
+                const Acc d = c - v[j];
+                peak = peak && d > tol;
+                below = below || d < -tol;
+            }
+            if (!peak) {
+                ok = ok && below;
+                continue;
+            }
+            if (found == 0 || c > v0) {
+                v1 = v0;
+                v0 = c;
+                k0 = i;
+            } else if (found == 1 || c > v1) {
+                v1 = c;
+            }
+            ++found;
+        }
+        opiv_vector out{ 0.f, 0.f, 0.f, 0.f, 0.f };
+        int32_t code = -1;
+        int px = W / 2, py = W / 2;
+        if (found >= 2) {
+            const Acc x = val[5 * k0 + (lane < 5 ? lane : 0)];
+            ok = ok && v0 - v1 > tol && (v1 > tol || v1 < -tol);
+            ok = __all_sync(0xffffffffu, ok && (x > tol || x < -tol));
+            const double lv = log((double)x);   // NaN where the reference's is
+            const double lc = __shfl_sync(0xffffffffu, lv, 0);
+            const double ll = __shfl_sync(0xffffffffu, lv, 1), lr = __shfl_sync(0xffffffffu, lv, 2);
+            const double lu = __shfl_sync(0xffffffffu, lv, 3), ld = __shfl_sync(0xffffffffu, lv, 4);
+            // the three quotients on three lanes: x offset, y offset, sn
+            const double lo = lane == 1 ? lu : ll, hi = lane == 1 ? ld : lr;
+            const double num = lane == 2 ? (double)v0 : lo - hi;
+            const double den = lane == 2 ? (double)v1 : 2.0 * (lo + hi - 2.0 * lc);
+            // a flatter peak than this magnifies the FP64 rounding too much
+            ok = __all_sync(0xffffffffu, ok && !(fabs(den) < 1e-8));
+            const double quot = num / den;
+            const int key = rs.key[k0];
+            px = key & m;
+            py = key >> lg;
+            const double lx = (double)px + __shfl_sync(0xffffffffu, quot, 0);
+            const double ly = (double)py + __shfl_sync(0xffffffffu, quot, 1);
+            const double sn = __shfl_sync(0xffffffffu, quot, 2);
+            const int mx = bx + W / 2, my = by + W / 2;
+            out.x = (float)mx;
+            out.y = (float)(p.img_h - my);
+            out.u = (float)((double)mx - ((double)bx + lx) - (double)ox);
+            out.v = (float)((double)my - ((double)by + ly) - (double)oy);
+            out.sn = v1 > 0 ? (float)sn : 0.f;
+            code = key | OPIV_PEAK_EXACT;
+        }
+        if (lane == 0) {
+            rs.ok = ok;
+            if (ok) {
+                if (p.out_vec) p.out_vec[w] = out;
+                if (p.out_peak) p.out_peak[w] = code;
+                if (p.out_disp) p.out_disp[w] = pack_disp(px - W / 2 + ox, py - W / 2 + oy);
+            }
+        }
+    }
+    __syncthreads();
+    const bool ok = rs.ok;
+    __syncthreads();   // read before the next window
+    return ok;
+}
+
 // scan range in plane coordinates (find_peaks on the plane or on its
 // centre view rect().dilate(0.5); rect.cpp:109-126)
 __device__ __forceinline__ void scan_range(int W, int limit, int& sy0, int& sy1, int& sx0, int& sx1)
@@ -288,18 +548,28 @@ __device__ __forceinline__ void scan_range(int W, int limit, int& sy0, int& sy1,
     sx1 = d0 + vw - 1;
 }
 
-template <typename PixT>
+// LIST: the windows of flag_list (the pass after the FP32 kernel), exact
+// sums first; otherwise every window in FP64.
+template <typename PixT, bool LIST>
 __global__ void __launch_bounds__(kThreads)
-piv_exact_kernel(const PivParams p, int W, int mode, int limit, bool use_list)
+piv_exact_kernel(const PivParams p, int W, int mode, int limit)
 {
     extern __shared__ double2 sm[];
     __shared__ int row_count[kMaxW];
     __shared__ int total_cand;
-    const int64_t nwork = use_list ? (int64_t)(*p.flag_count) : p.n_win;
+    const int64_t nwork = LIST ? (int64_t)(*p.flag_count) : p.n_win;
     int sy0, sy1, sx0, sx1;
     scan_range(W, limit, sy0, sy1, sx0, sx1);
     for (int64_t item = blockIdx.x; item < nwork; item += gridDim.x) {
-        const int64_t w = use_list ? (int64_t)p.flag_list[item] : item;
+        const int64_t w = LIST ? (int64_t)p.flag_list[item] : item;
+        if constexpr (LIST) {
+            __shared__ refine_shared rs;
+            if (item < p.flag_cap &&
+                refine_window<PixT>(p, w, W, mode, sy0, sy1, sx0, sx1,
+                                    p.flag_planes + (size_t)item * flag_record_floats(W),
+                                    reinterpret_cast<unsigned char*>(sm), rs))
+                continue;
+        }
         exact_window<PixT>(p, w, W, mode, sy0, sy1, sx0, sx1, sm, sm + W * W, row_count, &total_cand);
     }
 }
@@ -313,6 +583,7 @@ piv_exact_queue_kernel(const __grid_constant__ PivQueue q, int W, int mode, int 
     extern __shared__ double2 sm[];
     __shared__ int row_count[kMaxW];
     __shared__ int total_cand;
+    __shared__ refine_shared rs;
     const int64_t nwork = (int64_t)(*q.flag_count);
     int sy0, sy1, sx0, sx1;
     scan_range(W, limit, sy0, sy1, sx0, sx1);
@@ -324,14 +595,19 @@ piv_exact_queue_kernel(const __grid_constant__ PivQueue q, int W, int mode, int 
             if (q.first_win[mid] <= g) lo = mid;
             else hi = mid - 1;
         }
-        exact_window<PixT>(q.items[lo], (int64_t)(g - q.first_win[lo]), W, mode, sy0, sy1, sx0, sx1,
-                           sm, sm + W * W, row_count, &total_cand);
+        const PivParams& p = q.items[lo];
+        const int64_t w = (int64_t)(g - q.first_win[lo]);
+        if (item < p.flag_cap &&
+            refine_window<PixT>(p, w, W, mode, sy0, sy1, sx0, sx1,
+                                p.flag_planes + (size_t)item * flag_record_floats(W),
+                                reinterpret_cast<unsigned char*>(sm), rs))
+            continue;
+        exact_window<PixT>(p, w, W, mode, sy0, sy1, sx0, sx1, sm, sm + W * W, row_count, &total_cand);
     }
 }
 
-template <typename PixT>
-cudaError_t launch_t(const PivParams& p, int w, int mode, int limit, bool use_list, int blocks,
-                     cudaStream_t s)
+template <typename PixT, bool LIST>
+cudaError_t launch_t(const PivParams& p, int w, int mode, int limit, int blocks, cudaStream_t s)
 {
     const size_t smem = 2 * sizeof(double2) * (size_t)w * w;
     // the opt-in limit for the largest window, once per device
@@ -340,13 +616,13 @@ cudaError_t launch_t(const PivParams& p, int w, int mode, int limit, bool use_li
     cudaGetDevice(&dev);
     const uint64_t bit = 1ull << (dev & 63);
     if (!(attr_done.load() & bit)) {
-        const cudaError_t e = cudaFuncSetAttribute(piv_exact_kernel<PixT>,
+        const cudaError_t e = cudaFuncSetAttribute(piv_exact_kernel<PixT, LIST>,
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                    (int)(2 * sizeof(double2) * 64 * 64));
         if (e != cudaSuccess) return e;
         attr_done.fetch_or(bit);
     }
-    piv_exact_kernel<PixT><<<blocks, kThreads, smem, s>>>(p, w, mode, limit, use_list);
+    piv_exact_kernel<PixT, LIST><<<blocks, kThreads, smem, s>>>(p, w, mode, limit);
     return cudaGetLastError();
 }
 
@@ -501,10 +777,17 @@ cudaError_t launch_piv_exact(const PivParams& p, int w, int dtype, int mode, int
 {
     if (!exact_supports(w) || blocks <= 0) return cudaErrorInvalidValue;
     switch (dtype) {
-    case kU8: return launch_t<uint8_t>(p, w, mode, limit, use_list, blocks, s);
-    case kU16: return launch_t<uint16_t>(p, w, mode, limit, use_list, blocks, s);
-    case kF32: return launch_t<float>(p, w, mode, limit, use_list, blocks, s);
-    case kF64: return launch_t<double>(p, w, mode, limit, use_list, blocks, s);
+    case kU8:
+        return use_list ? launch_t<uint8_t, true>(p, w, mode, limit, blocks, s)
+                        : launch_t<uint8_t, false>(p, w, mode, limit, blocks, s);
+    case kU16:
+        return use_list ? launch_t<uint16_t, true>(p, w, mode, limit, blocks, s)
+                        : launch_t<uint16_t, false>(p, w, mode, limit, blocks, s);
+    case kF32:
+        return use_list ? launch_t<float, true>(p, w, mode, limit, blocks, s)
+                        : launch_t<float, false>(p, w, mode, limit, blocks, s);
+    case kF64:   // the per-window API's double windows: never a list
+        return use_list ? cudaErrorInvalidValue : launch_t<double, false>(p, w, mode, limit, blocks, s);
     default: return cudaErrorInvalidValue;
     }
 }

@@ -448,6 +448,7 @@ __device__ __forceinline__ void fp32_task(const PivParams& p, const int task, fl
         const float lyu = __shfl_sync(0xffffffffu, lg, 4, W);
         const float lydd = __shfl_sync(0xffffffffu, lg, 5, W);
 
+        int slot = -1;
         if (valid && gl == 0) {
             const bool has2 = t1 > kNegInf;
             bool certain;
@@ -496,9 +497,18 @@ __device__ __forceinline__ void fp32_task(const PivParams& p, const int task, fl
             if (p.out_disp)
                 p.out_disp[w] = has2 ? pack_disp(px - W / 2 + ox, py - W / 2 + oy) : pack_disp(ox, oy);
             if (!certain && p.flag_list) {
-                const unsigned int slot = atomicAdd(p.flag_count, 1u);
-                p.flag_list[slot] = (int32_t)w + p.flag_base;
+                const unsigned int at = atomicAdd(p.flag_count, 1u);
+                p.flag_list[at] = (int32_t)w + p.flag_base;
+                if (at < (unsigned int)p.flag_cap) slot = (int)at;
             }
+        }
+        // a flagged window hands its plane on (each lane its own column)
+        if (!PLANES) slot = __shfl_sync(0xffffffffu, slot, 0, W);
+        if (!PLANES && slot >= 0) {
+            float* rec = p.flag_planes + (size_t)slot * flag_record_floats(W);
+#pragma unroll 4
+            for (int y = 0; y < W; ++y) rec[((y + W / 2) & (W - 1)) * W + xs] = S[tix<W>(y, gl)].x;
+            if (gl == 0) rec[N] = dlt;
         }
     }
 }

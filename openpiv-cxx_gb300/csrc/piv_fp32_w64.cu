@@ -181,6 +181,7 @@ __device__ __forceinline__ void w64_task(const PivParams& p, const int blk)
     __shared__ float rv0[kWarps], rv1[kWarps], ru[kWarps];
     __shared__ int rk[kWarps];
     __shared__ float sped[2];
+    __shared__ int s_slot[2];
 
     const int t = threadIdx.x;
     const int w0 = 2 * blk;
@@ -355,6 +356,7 @@ __device__ __forceinline__ void w64_task(const PivParams& p, const int blk)
         if (lane == 0) { rv0[wp] = t0; rv1[wp] = t1; rk[wp] = key; ru[wp] = umax; }
         __syncthreads();
         if (t == 0) {
+            s_slot[h] = -1;
             float g0 = kNegInf64, g1 = kNegInf64, gu = kNegInf64;
             int gk = 0x7fffffff;
             for (int i = 0; i < kWarps; ++i) {
@@ -410,12 +412,27 @@ __device__ __forceinline__ void w64_task(const PivParams& p, const int blk)
                                               : pack_disp(ox, oy);
                 }
                 if (!certain && p.flag_list) {
-                    const unsigned int slot = atomicAdd(p.flag_count, 1u);
-                    p.flag_list[slot] = (int32_t)w + p.flag_base;
+                    const unsigned int at = atomicAdd(p.flag_count, 1u);
+                    p.flag_list[at] = (int32_t)w + p.flag_base;
+                    if (at < (unsigned int)p.flag_cap) s_slot[h] = (int)at;
                 }
             }
         }
         __syncthreads();
+    }
+    // flagged windows hand their planes on
+    if (!PLANES && (s_slot[0] & s_slot[1]) >= 0) {
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {
+            if (s_slot[h] < 0) continue;
+            float* rec = p.flag_planes + (size_t)s_slot[h] * flag_record_floats(W);
+            for (int i = t; i < N; i += kThreads) {
+                const float2 v = T1[at(((i >> 6) + W / 2) & (W - 1), (i + W / 2) & (W - 1))];
+                rec[i] = h ? v.y : v.x;
+            }
+            if (t == 0) rec[N] = dlt;
+        }
+        __syncthreads();   // T1 and the slots are the next task's
     }
 }
 

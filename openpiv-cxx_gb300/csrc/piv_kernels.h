@@ -30,6 +30,11 @@ struct PivParams {
     unsigned int* flag_count = nullptr;
     int32_t* flag_list = nullptr;
     int32_t flag_base = 0;             // added to a flagged window's index (a queue's list)
+    // planes of the first flag_cap flagged windows, by their place in the
+    // list: flag_record_floats(W) floats each, the quadrant-swapped FP32
+    // plane and then its error bound (refine_window in piv_exact.cu)
+    int32_t flag_cap = 0;
+    float* flag_planes = nullptr;
     float kappa = 16.f;                // FP32 error-bound factor
     // debug / per-window API outputs
     float* planes = nullptr;           // FP32 kernel: n_win * W * W (mean-free part)
@@ -50,6 +55,10 @@ struct PivParams {
     int32_t* out_disp = nullptr;       // this pass's integer displacements (may be null)
     int* status = nullptr;             // tensor-core kernel: set to 1 if an MMA wait gave up
 };
+
+// Floats of a flagged window's record: the plane, its error bound, padding
+// to 16 bytes.
+__host__ __device__ constexpr int flag_record_floats(int w) { return w * w + 4; }
 
 // Tensor-core DFT-GEMM kernels (piv_tc.cu): 16, 32, 48 and 64 px windows
 // (32: piv_tc_kernel.cuh; the others: piv_tcg_kernel.cuh), u8/u16 frames,
@@ -152,7 +161,7 @@ struct PivQueue {
     const int32_t* flag_list = nullptr;
 };
 static_assert(kQueueMaxItems <= 256, "task_item holds pair numbers in one byte");
-static_assert(sizeof(PivParams) == 208, "descriptor size (queue parameter space)");
+static_assert(sizeof(PivParams) == 224, "descriptor size (queue parameter space)");
 static_assert(sizeof(PivParams) % 16 == 0, "descriptors are copied in 16-byte words");
 // tasks of a pair of n_win windows in the queue of window size w
 inline int fp32_queue_tasks(int w, int64_t n_win)
