@@ -1,23 +1,44 @@
 // piv_fp32_w64.cu -- fused FP32 PIV kernel for 64 x 64 windows (sm_103a).
 //
 // A 64-point row does not fit one lane's registers next to everything else,
-// so this kernel keeps the pair's spectra in shared memory: one CTA of 256
-// threads per pair of windows, two padded 64 x 67 float2 tiles.  The steps
-// and the formulas are those of the 16/32 kernel (piv_fp32.cuh):
-//   z = a + i b; 2-D FFT (rows, then columns) as two radix-8 decimation-
-//   in-frequency passes over the tile (64 = 8^2; outputs in base-8 digit-
-//   reversed order, absorbed in the indexing);
-//   bank-conflict-free tile layout: column c of a row sits at c + 2 (c/16)
-//   and rows are 71 float2 apart, so sixteen threads reading sixteen
-//   neighbouring rows, sixteen neighbouring columns, or the sixteen columns
-//   of a digit-reversed block all hit distinct banks;
-//   4 conj(P) = (2 Im(Z Zm), |Z|^2 - |Zm|^2) with Zm = Z[-k] (P = B conj A,
-//   fft.h:188-227), REAL mode's zeroed spectrum row 0, row W/2, column 0
-//   (fft.h:166-183), DC product dropped and the pedestal added back;
-//   Q = conj(4 P1) + i conj(4 P2), one forward 2-D FFT -> both planes;
-//   find_peaks(plane, 2, 1) (image_utils.impl.h:42-74) as a block scan and
-//   reduction; fit_simple_gaussian (impl:77-101); vector of main.cpp:220-236;
-//   the same certification and hand-off to the exact kernel.
+// so one CTA of 256 threads takes a pair of windows through one 64 x 64
+// float2 tile in shared memory.  z = a + i b of a window is transformed by
+// radix-8 decimation-in-frequency passes (64 = 8^2), each thread taking two
+// 8-point butterflies a pass; a pass's output goes back where its input came
+// from, and the base-8 digit reversal that this leaves is absorbed in which
+// rows or columns the next pass reads:
+//   1  pixels from the frames, columns 8-point                 -> tile
+//   2  columns 8-point;  3  rows 8-point                       tile -> tile
+//   4  rows 8-point in registers, for both bins k and -k of the unpack:
+//      a thread takes the butterflies of spectrum row k_y and of row -k_y, so
+//      4 conj(P) = (2 Im(Z Zm), |Z|^2 - |Zm|^2) with Zm = Z[-k]
+//      (P = B conj A, fft.h:188-227) needs nothing of another thread's.
+//      The first window's products wait in 16 registers while the second
+//      window goes through 1 to 4 in the same tile; then
+//      Q = conj(4 P1) + i conj(4 P2) is formed at k and -k, and since a
+//      butterfly's eight bins are what the inverse's first row pass takes,
+//      that pass runs on them at once                          -> tile
+//   5  rows 8-point;  6, 7  columns 8-point: plane 1 + i plane 2, natural order
+// (one forward 2-D FFT of Q gives both planes).  REAL mode zeroes spectrum
+// row 0, row W/2 and column 0 (fft.h:166-183), COMPLEX the DC bin, whose
+// pedestal is added back.  find_peaks(plane, 2, 1) (image_utils.impl.h:42-74)
+// is a scan of both planes at once, the fit (impl:77-101), the vector of
+// main.cpp:220-236 and the certification run on one warp per window.
+//
+// The tile is transposed: its lines are image columns x (spectrum columns
+// k_x), 65 float2 apart, elements along a line are y.  Sixteen threads
+// reading sixteen neighbouring lines, sixteen neighbouring elements, or step
+// 4's mirrored elements (two reversed groups of eight) all hit distinct
+// banks; a warp's pixel loads are 32 neighbours of one image row; and an
+// element's offset from its butterfly's first is a compile-time constant.
+//
+// 2048 x 2048, u16, step 16 (15,625 windows): 464 us with two tiles, seventeen
+// trips through shared memory and a serial fit on one thread, 240 us with
+// this (13,300 warp instructions a window where it took 21,600).  Packed FP32
+// (add2, sub2, fma2) took 268 to 242 us of that: the kernel is bound by issue
+// slots (about 75 % busy), then by shared-memory wavefronts (65 %), so one
+// instruction for both components pays although the FP32 pipe's rate is the
+// same.  One tile (33 KB) and 64 registers let four CTAs share an SM.
 
 #include <atomic>
 #include <cstdint>
@@ -32,9 +53,10 @@ namespace w64 {
 
 constexpr int W = 64;
 constexpr int N = W * W;
-constexpr int LD = W + 7;            // row stride (float2), odd: rows fall on distinct banks
+constexpr int LD = W + 1;            // row stride (float2), odd: rows fall on distinct banks
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
+constexpr int kCtasPerSm = 4;
 // certification thresholds: as the 16 / 32 px kernel (piv_fp32.cuh)
 constexpr float kFitTol = 6e-5f;
 constexpr float kSnTol = 6e-6f;
@@ -48,74 +70,217 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 w)
     return make_float2(fmaf(a.x, w.x, -a.y * w.y), fmaf(a.x, w.y, a.y * w.x));
 }
 
-// offset of column c inside a row: two pad elements after every 16 columns
-__device__ __forceinline__ int pos(int c) { return c + 2 * (c >> 4); }
+// Packed FP32 pairs (one instruction for both components; each rounds as the
+// scalar one does).
+__device__ __forceinline__ float2 add2(float2 a, float2 b)
+{
+    float2 d;
+    asm("{ .reg .b64 x, y; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; add.rn.f32x2 x, x, y; mov.b64 {%0, %1}, x; }"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+__device__ __forceinline__ float2 sub2(float2 a, float2 b)
+{
+    float2 d;
+    asm("{ .reg .b64 x, y; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; sub.rn.f32x2 x, x, y; mov.b64 {%0, %1}, x; }"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
+{
+    float2 d;
+    asm("{ .reg .b64 x, y, z; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; mov.b64 z, {%6, %7}; "
+        "fma.rn.f32x2 x, x, y, z; mov.b64 {%0, %1}, x; }"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
 
 // In-place forward 8-point DFT, natural order in and out.
 __device__ __forceinline__ void dft8(float2* x)
 {
     constexpr float r = 0.70710678118654752f;   // cos(pi/4)
-    const float2 a0 = make_float2(x[0].x + x[4].x, x[0].y + x[4].y), a1 = make_float2(x[0].x - x[4].x, x[0].y - x[4].y);
-    const float2 a2 = make_float2(x[2].x + x[6].x, x[2].y + x[6].y), a3 = make_float2(x[2].x - x[6].x, x[2].y - x[6].y);
-    const float2 a4 = make_float2(x[1].x + x[5].x, x[1].y + x[5].y), a5 = make_float2(x[1].x - x[5].x, x[1].y - x[5].y);
-    const float2 a6 = make_float2(x[3].x + x[7].x, x[3].y + x[7].y), a7 = make_float2(x[3].x - x[7].x, x[3].y - x[7].y);
+    const float2 a0 = add2(x[0], x[4]), a1 = sub2(x[0], x[4]), a2 = add2(x[2], x[6]), a3 = sub2(x[2], x[6]);
+    const float2 a4 = add2(x[1], x[5]), a5 = sub2(x[1], x[5]), a6 = add2(x[3], x[7]), a7 = sub2(x[3], x[7]);
     // even outputs: 4-point DFT of (a0, a4, a2, a6)
-    const float2 e0 = make_float2(a0.x + a2.x, a0.y + a2.y), e1 = make_float2(a0.x - a2.x, a0.y - a2.y);
-    const float2 e2 = make_float2(a4.x + a6.x, a4.y + a6.y), e3 = make_float2(a4.x - a6.x, a4.y - a6.y);
-    x[0] = make_float2(e0.x + e2.x, e0.y + e2.y);
-    x[4] = make_float2(e0.x - e2.x, e0.y - e2.y);
+    const float2 e0 = add2(a0, a2), e1 = sub2(a0, a2), e2 = add2(a4, a6), e3 = sub2(a4, a6);
+    x[0] = add2(e0, e2);
+    x[4] = sub2(e0, e2);
     x[2] = make_float2(e1.x + e3.y, e1.y - e3.x);   // e1 - i e3
     x[6] = make_float2(e1.x - e3.y, e1.y + e3.x);   // e1 + i e3
     // odd outputs: 4-point DFT of (a1, a5 w, -i a3, a7 w^3), w = exp(-i pi/4)
     const float2 b1 = make_float2((a5.x + a5.y) * r, (a5.y - a5.x) * r);
     const float2 b3 = make_float2((a7.y - a7.x) * r, -(a7.x + a7.y) * r);
     const float2 o0 = make_float2(a1.x + a3.y, a1.y - a3.x), o1 = make_float2(a1.x - a3.y, a1.y + a3.x);
-    const float2 o2 = make_float2(b1.x + b3.x, b1.y + b3.y), o3 = make_float2(b1.x - b3.x, b1.y - b3.y);
-    x[1] = make_float2(o0.x + o2.x, o0.y + o2.y);
-    x[5] = make_float2(o0.x - o2.x, o0.y - o2.y);
+    const float2 o2 = add2(b1, b3), o3 = sub2(b1, b3);
+    x[1] = add2(o0, o2);
+    x[5] = sub2(o0, o2);
     x[3] = make_float2(o1.x + o3.y, o1.y - o3.x);   // o1 - i o3
     x[7] = make_float2(o1.x - o3.y, o1.y + o3.x);   // o1 + i o3
 }
 
-// One radix-8 DIF pass over all 64 lines of tile T (rows when ROWS, else
-// columns).  FIRST: butterfly j takes elements j + 8 m and scales output m
-// by tw[j m] = exp(-2 pi i j m / 64); second pass: butterfly j takes
-// elements 8 j + m, no twiddles.  After both passes bin k0 + 8 k1 of a line
-// sits at 8 k0 + k1.  Neighbouring threads take neighbouring lines and the
-// same butterfly, so a warp's twiddles are one broadcast.
-template <bool ROWS, bool FIRST>
-__device__ __forceinline__ void dif8_pass(float2* T, const float2* tw)
+// An 8-point butterfly over tile elements T[0], T[S], .. T[7 S].
+template <int S>
+__device__ __forceinline__ void load8(const float2* T, float2 (&x)[8])
 {
 #pragma unroll
-    for (int it = 0; it < 64 * 8 / kThreads; ++it) {
-        const int k = (int)threadIdx.x + it * kThreads;
-        const int line = k & 63, j = k >> 6;
-        const int base = FIRST ? j : 8 * j, es = FIRST ? 8 : 1;
-        auto el = [&](int e) -> float2& { return ROWS ? T[line * LD + pos(e)] : T[e * LD + pos(line)]; };
-        float2 x[8];
+    for (int m = 0; m < 8; ++m) x[m] = T[m * S];
+}
+template <int S>
+__device__ __forceinline__ void store8(float2* T, const float2 (&x)[8])
+{
 #pragma unroll
-        for (int m = 0; m < 8; ++m) x[m] = el(base + m * es);
-        dft8(x);
-        if (FIRST) {
+    for (int m = 0; m < 8; ++m) T[m * S] = x[m];
+}
+// Output m of a first pass's butterfly j is scaled by exp(-2 pi i j m / 64):
+// row j of the table, in four 16-byte loads (a warp's lanes share j).
+constexpr int kTwRow = 8;
+struct twiddles {
+    float4 w[4];
+    __device__ __forceinline__ twiddles(const float2* tw, int j)
+    {
+        const float4* q = reinterpret_cast<const float4*>(tw + j * kTwRow);
 #pragma unroll
-            for (int m = 1; m < 8; ++m) x[m] = cmul(x[m], tw[j * m]);
+        for (int i = 0; i < 4; ++i) w[i] = q[i];
+    }
+    __device__ __forceinline__ void scale(float2 (&x)[8]) const
+    {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (i > 0) x[2 * i] = cmul(x[2 * i], make_float2(w[i].x, w[i].y));
+            x[2 * i + 1] = cmul(x[2 * i + 1], make_float2(w[i].z, w[i].w));
         }
+    }
+};
+
+// Passes over the whole tile: along its lines (lanes take lines, so a
+// warp's j is uniform) or across them, elements 8 j + m or j + 8 m.
+template <bool ALONG, bool BLOCK, bool TWIDDLE>
+__device__ __forceinline__ void pass8(float2* T, const float2* tw)
+{
+    const int line = (int)threadIdx.x & 63;
 #pragma unroll
-        for (int m = 0; m < 8; ++m) el(base + m * es) = x[m];
+    for (int it = 0; it < 2; ++it) {
+        const int j = ((int)threadIdx.x >> 6) + 4 * it;
+        float2 x[8];
+        constexpr int E = ALONG ? 1 : LD, L = ALONG ? LD : 1;   // element and line strides
+        float2* e = T + line * L + (BLOCK ? 8 * j : j) * E;
+        load8<(BLOCK ? 1 : 8) * E>(e, x);
+        dft8(x);
+        if (TWIDDLE) twiddles(tw, j).scale(x);
+        store8<(BLOCK ? 1 : 8) * E>(e, x);
     }
     __syncthreads();
 }
 
-__device__ __forceinline__ void fft2d(float2* T, const float2* tw)
+// ---- the unpack's pairs of bins ------------------------------------------------
+// A thread's butterflies: A at spectrum row ky, j (bins kx = j + 8 m) and B at
+// row -ky, -j.  Bin m of A mirrors bin 7 - m of B, or (8 - m) & 7 where j = 0.
+// Threads of warps 0 .. 5 take j = 1, 2, 3 and every row; warp 6 takes j = 0
+// and warp 7 j = 4 with one row of each mirrored two (tile elements 1 .. 3,
+// 36 .. 39, 8 .. 31), whose lane 0 holds the two that mirror themselves,
+// ky = 0 (A) and W/2 (B).  In the tile's digit-reversed order -ky of the eight
+// elements 8 g .. 8 g + 7 are the eight of group 8 - g, reversed (group 0:
+// its own, reversed but for the first).
+struct pair_slot {
+    float im, d;   // 2 Im(Z Zm), |Z|^2 - |Zm|^2 at A's bin; at B's bin im, -d
+};
+__device__ __forceinline__ pair_slot product(float2 z, float2 m)
 {
-    dif8_pass<true, true>(T, tw);
-    dif8_pass<true, false>(T, tw);
-    dif8_pass<false, true>(T, tw);
-    dif8_pass<false, false>(T, tw);
+    pair_slot s;
+    s.im = 2.f * fmaf(z.x, m.y, z.y * m.x);
+    s.d = fmaf(z.x, z.x, fmaf(z.y, z.y, -fmaf(m.x, m.x, m.y * m.y)));
+    return s;
+}
+// Q = conj(4 P1) + i conj(4 P2) at A's bin and at its mirror
+__device__ __forceinline__ float2 q_at(pair_slot a, pair_slot b) { return make_float2(a.im - b.d, a.d + b.im); }
+__device__ __forceinline__ float2 q_mirror(pair_slot a, pair_slot b) { return make_float2(a.im + b.d, b.im - a.d); }
+
+__device__ __forceinline__ void pick(float2& a, float2& b, float2& c, bool rotate)
+{   // (a, b, c) -> (c', a', b') = (b, c, a) when rotating
+    const float2 x = a, y = b, z = c;
+    a = rotate ? y : x;
+    b = rotate ? z : y;
+    c = rotate ? x : z;
+}
+// Lane 0 of warp 7: both rows mirror themselves with 7 - m; exchanging
+// quarters makes its pairs those of the other threads, (X[m], Y[7 - m]) with
+// X = A[0..3], B[0..3] and Y = B[4..7], A[4..7].
+__device__ __forceinline__ void to_pairs(float2 (&A)[8], float2 (&B)[8], bool self)
+{
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        pick(A[4 + i], B[i], B[4 + i], self);   // A[4+i] <- B[i], B[i] <- B[4+i], B[4+i] <- A[4+i]
+    }
+}
+__device__ __forceinline__ void from_pairs(float2 (&A)[8], float2 (&B)[8], bool self)
+{
+#pragma unroll
+    for (int i = 0; i < 4; ++i) pick(B[4 + i], B[i], A[4 + i], self);   // the inverse exchange
 }
 
-// position in a transformed tile of spectrum bin (ky, kx) / plane (y, x)
-__device__ __forceinline__ int at(int r, int c) { return dr(r) * LD + pos(dr(c)); }
+// Products of a window's bins, one slot per pair.
+__device__ __forceinline__ void products(float2 (&A)[8], float2 (&B)[8], int j, bool self, pair_slot (&s)[8])
+{
+    if (j != 0) {
+        if (j == 4) to_pairs(A, B, self);
+#pragma unroll
+        for (int m = 0; m < 8; ++m) s[m] = product(A[m], B[7 - m]);
+    } else if (!self) {
+#pragma unroll
+        for (int m = 0; m < 8; ++m) s[m] = product(A[m], B[(8 - m) & 7]);
+    } else {   // rows 0 and W/2 themselves: bins 0 and 4 are their own mirrors (d = 0), kept in one slot
+        s[0] = pair_slot{ product(A[0], A[0]).im, product(A[4], A[4]).im };
+        s[4] = pair_slot{ product(B[0], B[0]).im, product(B[4], B[4]).im };
+#pragma unroll
+        for (int m = 1; m < 4; ++m) {
+            s[m] = product(A[m], A[8 - m]);
+            s[4 + m] = product(B[m], B[8 - m]);
+        }
+    }
+}
+// Q at all bins of the two butterflies from both windows' products.
+__device__ __forceinline__ void pack(const pair_slot (&s1)[8], const pair_slot (&s2)[8], int j, bool self,
+                                     float2 (&A)[8], float2 (&B)[8])
+{
+    if (j != 0) {
+#pragma unroll
+        for (int m = 0; m < 8; ++m) {
+            A[m] = q_at(s1[m], s2[m]);
+            B[7 - m] = q_mirror(s1[m], s2[m]);
+        }
+        if (j == 4) from_pairs(A, B, self);
+    } else if (!self) {
+#pragma unroll
+        for (int m = 0; m < 8; ++m) {
+            A[m] = q_at(s1[m], s2[m]);
+            B[(8 - m) & 7] = q_mirror(s1[m], s2[m]);
+        }
+    } else {
+        A[0] = make_float2(s1[0].im, s2[0].im);
+        A[4] = make_float2(s1[0].d, s2[0].d);
+        B[0] = make_float2(s1[4].im, s2[4].im);
+        B[4] = make_float2(s1[4].d, s2[4].d);
+#pragma unroll
+        for (int m = 1; m < 4; ++m) {
+            A[m] = q_at(s1[m], s2[m]);
+            A[8 - m] = q_mirror(s1[m], s2[m]);
+            B[m] = q_at(s1[4 + m], s2[4 + m]);
+            B[8 - m] = q_mirror(s1[4 + m], s2[4 + m]);
+        }
+    }
+}
+
+// Pixels a + i b to float, exactly (8/16-bit: into the mantissa of 2^23).
+template <typename PixT>
+__device__ __forceinline__ float2 widen(PixT a, PixT b)
+{
+    if constexpr (sizeof(PixT) <= 2)
+        return sub2(make_float2(__uint_as_float(0x4B000000u | a), __uint_as_float(0x4B000000u | b)),
+                    make_float2(8388608.f, 8388608.f));
+    else
+        return make_float2((float)a, (float)b);
+}
 
 __device__ __forceinline__ void window_origin(const PivParams& p, int w, int& bx, int& by)
 {
@@ -129,6 +294,14 @@ __device__ __forceinline__ void window_origin(const PivParams& p, int w, int& bx
     }
 }
 
+// a three-source max and a max
+__device__ __forceinline__ float max4(float a, float b, float c, float d)
+{
+    float m;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(fmaxf(c, d)));
+    return m;
+}
+
 // Running top-2 of strict 4-neighbour maxima (find_peaks) plus the largest
 // value whose strict-maximum decision is within dlt of flipping.
 struct Top2 {
@@ -137,30 +310,30 @@ struct Top2 {
     __device__ __forceinline__ void init()
     {
         t0 = t1 = umax = kNegInf64;
-        key = 0x7fffffff;
+        key = 0;
     }
     __device__ __forceinline__ void add(float c, float m, float dlt, int k)
     {
         const float dd = m - c;
-        if (fabsf(dd) <= dlt) umax = fmaxf(umax, c);
-        if (dd < 0.f) {
-            if (c > t0) { t1 = t0; t0 = c; key = k; }
-            else t1 = fmaxf(t1, c);
-        }
+        umax = fabsf(dd) <= dlt ? fmaxf(umax, c) : umax;
+        const float v = dd < 0.f ? c : kNegInf64;
+        t1 = fmaxf(t1, fminf(t0, v));
+        key = v > t0 ? k : key;
+        t0 = fmaxf(t0, v);
+    }
+    // with the lanes o away (ties to the lowest row-major index)
+    __device__ __forceinline__ void merge(int o)
+    {
+        const float o0 = __shfl_xor_sync(0xffffffffu, t0, o);
+        const float o1 = __shfl_xor_sync(0xffffffffu, t1, o);
+        const int ok = __shfl_xor_sync(0xffffffffu, key, o);
+        const bool take = (o0 > t0) || (o0 == t0 && ok < key);
+        t1 = fmaxf(fmaxf(t1, o1), fminf(t0, o0));
+        key = take ? ok : key;
+        t0 = fmaxf(t0, o0);
+        umax = fmaxf(umax, __shfl_xor_sync(0xffffffffu, umax, o));
     }
 };
-
-__device__ __forceinline__ float block_sum(float v, float* red)
-{
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    float s = 0.f;
-    for (int i = 0; i < kWarps; ++i) s += red[i];
-    __syncthreads();
-    return s;
-}
 
 extern __shared__ float2 w64_dyn_smem[];
 
@@ -173,271 +346,281 @@ __device__ __forceinline__ void w64_task(const PivParams& p, const int blk)
     constexpr int SY0 = D0 + 1, SY1 = D0 + VW - 2;
     constexpr int SX0 = D0 + 1, SX1 = D0 + VW - 1;
 
-    float2* sm = w64_dyn_smem;
-    float2* T1 = sm;                  // first window, then Q, then both planes
-    float2* T2 = sm + W * LD;         // second window
-    __shared__ float2 tw[64];
-    __shared__ float red[kWarps * 4];
-    __shared__ float rv0[kWarps], rv1[kWarps], ru[kWarps];
-    __shared__ int rk[kWarps];
-    __shared__ float sped[2];
-    __shared__ int s_slot[2];
+    float2* T = w64_dyn_smem;
+    __shared__ __align__(16) float2 tw[8 * kTwRow];
+    __shared__ float s_energy[kWarps];
+    __shared__ __align__(16) Top2 s_top[2][kWarps];
+    __shared__ float s_ped[2];
 
-    const int t = threadIdx.x;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int w0 = 2 * blk;
     if (w0 >= (int)p.n_win) return;
-    const int w1 = w0 + 1;
-    const bool valid1 = w1 < (int)p.n_win;
-    if (t < 64) tw[t] = make_float2(c_tw.re[t], c_tw.im[t]);
-
-    const PixT* fa = reinterpret_cast<const PixT*>(p.fa);
-    const PixT* fb = reinterpret_cast<const PixT*>(p.fb);
-    const size_t pitch = p.pitch / sizeof(PixT);
-
-    // ---- extract, widen, energies (and the exact pedestal for the batch API)
-    int bx0, by0, bx1 = 0, by1 = 0, ox0, oy0, ox1 = 0, oy1 = 0;
-    window_origin(p, w0, bx0, by0);
-    b_offset(p, W, bx0, by0, ox0, oy0);
-    if (valid1) {
-        window_origin(p, w1, bx1, by1);
-        b_offset(p, W, bx1, by1, ox1, oy1);
-    }
-    float e0 = 0.f, e1 = 0.f;
-    double sa0 = 0.0, sb0 = 0.0, sa1 = 0.0, sb1 = 0.0;
-    // pixels widen straight to float (exact for 8/16-bit frames); doubles
-    // only for the per-window API's exact pedestal (PLANES, double frames)
-    for (int i = t; i < N; i += kThreads) {
-        const int y = i >> 6, x = i & 63;
-        const PixT pa0 = __ldg(fa + (size_t)(by0 + y) * pitch + bx0 + x);
-        const PixT pb0 = __ldg(fb + (size_t)(by0 + oy0 + y) * pitch + bx0 + ox0 + x);
-        PixT pa1 = PixT(0), pb1 = PixT(0);
-        if (valid1) {
-            pa1 = __ldg(fa + (size_t)(by1 + y) * pitch + bx1 + x);
-            pb1 = __ldg(fb + (size_t)(by1 + oy1 + y) * pitch + bx1 + ox1 + x);
-        }
-        const float2 z0 = make_float2((float)pa0, (float)pb0), z1 = make_float2((float)pa1, (float)pb1);
-        T1[y * LD + pos(x)] = z0;
-        T2[y * LD + pos(x)] = z1;
-        e0 = fmaf(z0.x, z0.x, fmaf(z0.y, z0.y, e0));
-        e1 = fmaf(z1.x, z1.x, fmaf(z1.y, z1.y, e1));
-        if (PLANES) {
-            sa0 += (double)pa0;
-            sb0 += (double)pb0;
-            sa1 += (double)pa1;
-            sb1 += (double)pb1;
-        }
-    }
-    e0 = block_sum(e0, red);
-    e1 = block_sum(e1, red);
-    if (PLANES) {
-        const double s[4] = { sa0, sb0, sa1, sb1 };
-        double tot[4];
-        for (int c = 0; c < 4; ++c) {
-            double v = s[c];
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            __syncthreads();
-            if ((t & 31) == 0) reinterpret_cast<double*>(red)[t >> 5] = v;
-            __syncthreads();
-            double acc = 0.0;
-            for (int i = 0; i < kWarps; ++i) acc += reinterpret_cast<double*>(red)[i];
-            tot[c] = acc;
-            __syncthreads();
-        }
-        if (t == 0) {
-            p.peds[w0] = (MODE == kModeComplex) ? tot[0] * tot[1] : 0.0;
-            if (valid1) p.peds[w1] = (MODE == kModeComplex) ? tot[2] * tot[3] : 0.0;
-        }
+    const bool valid1 = w0 + 1 < (int)p.n_win;
+    if (t < 64) {
+        const int k = ((t >> 3) * (t & 7)) & 63;
+        tw[(t >> 3) * kTwRow + (t & 7)] = make_float2(c_tw.re[k], c_tw.im[k]);
     }
     __syncthreads();
 
-    // ---- forward transforms
-    fft2d(T1, tw);
-    fft2d(T2, tw);
-    if (t == 0) {   // DC bins: (sum a, sum b) of each window
-        const float2 d0 = T1[0], d1 = T2[0];
-        sped[0] = (MODE == kModeComplex) ? 4.f * d0.x * d0.y : 0.f;
-        sped[1] = (MODE == kModeComplex) ? 4.f * d1.x * d1.y : 0.f;
-    }
-    __syncthreads();
-    // zero the DC bin (COMPLEX) or the reference's unpacked-out set (REAL)
-    for (int i = t; i < N; i += kThreads) {
-        const int ky = i >> 6, kx = i & 63;
-        const bool zero = (MODE == kModeReal) ? (ky == 0 || ky == W / 2 || kx == 0)
-                                              : (ky == 0 && kx == 0);
-        if (zero) {
-            T1[at(ky, kx)] = make_float2(0.f, 0.f);
-            T2[at(ky, kx)] = make_float2(0.f, 0.f);
-        }
-    }
-    __syncthreads();
+    // the thread's pair of row butterflies (step 4)
+    const bool low = warp < 6;
+    const int j = low ? 1 + (warp >> 1) : (warp == 6 ? 0 : 4);
+    const int jb = (8 - j) & 7;
+    const int ca = low ? t & 63 : lane >= 4 && lane < 8 ? 32 + lane : lane;   // tile element of ky, of -ky
+    const bool self = !low && lane == 0;
+    const int cb = self ? dr(W / 2) : dr((W - dr(ca)) & (W - 1));
+    float2* const ea = T + 8 * j * LD + ca;
+    float2* const eb = T + 8 * jb * LD + cb;
 
-    // ---- products, packed: Q[ky][kx] = conj(4 P1) + i conj(4 P2), written
-    // in natural order (the next transform is a forward DIF again)
-    float2 q[N / kThreads];
+    float2 energy = make_float2(0.f, 0.f);
+    pair_slot first[8];
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+        float2 A[8], B[8];
+        if (h == 0 || valid1) {   // CTA-uniform
+            int bx, by, ox, oy;
+            window_origin(p, w0 + h, bx, by);
+            b_offset(p, W, bx, by, ox, oy);
+            const size_t pitch = p.pitch / sizeof(PixT);
+            const int x = t & 63;
+            const PixT* fa = reinterpret_cast<const PixT*>(p.fa) + (size_t)by * pitch + bx + x;
+            const PixT* fb = reinterpret_cast<const PixT*>(p.fb) + (size_t)(by + oy) * pitch + bx + ox + x;
+            double sa = 0.0, sb = 0.0;
 #pragma unroll
-    for (int n = 0; n < N / kThreads; ++n) {
-        const int i = t + n * kThreads;
-        const int ky = i >> 6, kx = i & 63;
-        const int mky = (W - ky) & (W - 1), mkx = (W - kx) & (W - 1);
-        const float2 z1 = T1[at(ky, kx)], m1 = T1[at(mky, mkx)];
-        const float2 z2 = T2[at(ky, kx)], m2 = T2[at(mky, mkx)];
-        const float im1 = 2.f * fmaf(z1.x, m1.y, z1.y * m1.x);
-        const float d1 = fmaf(z1.x, z1.x, fmaf(z1.y, z1.y, -fmaf(m1.x, m1.x, m1.y * m1.y)));
-        const float im2 = 2.f * fmaf(z2.x, m2.y, z2.y * m2.x);
-        const float d2 = fmaf(z2.x, z2.x, fmaf(z2.y, z2.y, -fmaf(m2.x, m2.x, m2.y * m2.y)));
-        q[n] = make_float2(im1 - d2, d1 + im2);
-    }
-    __syncthreads();
+            for (int it = 0; it < 2; ++it) {
+                const int j1 = (t >> 6) + 4 * it;   // rows j1 + 8 m of column x
+                const PixT *pa = fa + (size_t)j1 * pitch, *pb = fb + (size_t)j1 * pitch;
+                float2 v[8];
 #pragma unroll
-    for (int n = 0; n < N / kThreads; ++n) {
-        const int i = t + n * kThreads;
-        T1[(i >> 6) * LD + pos(i & 63)] = q[n];
+                for (int m = 0; m < 8; ++m) {
+                    const PixT a = __ldg(pa), b = __ldg(pb);
+                    pa += 8 * pitch;
+                    pb += 8 * pitch;
+                    v[m] = widen(a, b);
+                    energy = fma2(v[m], v[m], energy);
+                    if (PLANES) {   // the per-window API's exact pedestal (double frames)
+                        sa += (double)a;
+                        sb += (double)b;
+                    }
+                }
+                dft8(v);
+                twiddles(tw, j1).scale(v);
+                store8<8>(T + x * LD + j1, v);
+            }
+            if (PLANES) {
+                double* red = reinterpret_cast<double*>(&s_top[0][0]);   // 2 kWarps doubles, free until the scan
+                for (int o = 16; o > 0; o >>= 1) {
+                    sa += __shfl_xor_sync(0xffffffffu, sa, o);
+                    sb += __shfl_xor_sync(0xffffffffu, sb, o);
+                }
+                if (lane == 0) {
+                    red[2 * warp] = sa;
+                    red[2 * warp + 1] = sb;
+                }
+                __syncthreads();
+                if (t == 0) {
+                    sa = sb = 0.0;
+                    for (int i = 0; i < kWarps; ++i) {
+                        sa += red[2 * i];
+                        sb += red[2 * i + 1];
+                    }
+                    p.peds[w0 + h] = (MODE == kModeComplex) ? sa * sb : 0.0;
+                }
+            }
+            __syncthreads();
+            pass8<true, true, false>(T, tw);
+            pass8<false, false, true>(T, tw);
+            load8<LD>(ea, A);
+            load8<LD>(eb, B);
+            dft8(A);
+            dft8(B);
+            if (MODE == kModeComplex) {   // the DC bin (sum a, sum b)
+                if (self && j == 0) {
+                    s_ped[h] = 4.f * A[0].x * A[0].y;
+                    A[0] = make_float2(0.f, 0.f);
+                }
+            } else {                      // spectrum row 0, row W/2, column 0
+                const float2 zero = make_float2(0.f, 0.f);
+                // elements 0 and 4 are ky = 0 and W/2
+                const bool zero_a = (ca & ~4) == 0, zero_b = (cb & ~4) == 0;
+#pragma unroll
+                for (int m = 0; m < 8; ++m) {
+                    A[m] = zero_a || (m == 0 && j == 0) ? zero : A[m];
+                    B[m] = zero_b || (m == 0 && j == 0) ? zero : B[m];
+                }
+                if (t == 0) s_ped[h] = 0.f;
+            }
+        } else {
+#pragma unroll
+            for (int m = 0; m < 8; ++m) A[m] = B[m] = make_float2(0.f, 0.f);
+        }
+        if (h == 0) {
+            products(A, B, j, self, first);
+            __syncthreads();   // the tile is read: the second window's rows may come
+        } else {
+            pair_slot second[8];
+            products(A, B, j, self, second);
+            pack(first, second, j, self, A, B);
+            dft8(A);
+            dft8(B);
+            twiddles(tw, j).scale(A);
+            twiddles(tw, jb).scale(B);
+            store8<LD>(ea, A);
+            store8<LD>(eb, B);
+        }
+    }
+    {
+        float e = energy.x + energy.y;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+        if (lane == 0) s_energy[warp] = e;
     }
     __syncthreads();
-    fft2d(T1, tw);   // T1[at(y, x)] = plane1(y, x) + i plane2(y, x), 4x scaled
+    pass8<false, false, false>(T, tw);
+    pass8<true, true, true>(T, tw);
+    pass8<true, false, false>(T, tw);
 
-    const float dlt = p.kappa * 5.9604645e-8f * 2.f * (float)N * (e0 + e1);
-    const int lane = t & 31, wp = t >> 5;
+    // T[x * LD + y] = plane1(y, x) + i plane2(y, x), 4x scaled, before
+    // the quadrant swap
+    auto cell = [&](int ys, int xs) -> float2 {   // by swapped-plane coordinates
+        return T[((xs + W / 2) & (W - 1)) * LD + ((ys + W / 2) & (W - 1))];
+    };
+    float total = 0.f;
+#pragma unroll
+    for (int i = 0; i < kWarps; ++i) total += s_energy[i];
+    const float dlt = p.kappa * 5.9604645e-8f * 2.f * (float)N * total;
+
+    if (PLANES)
+        for (int h = 0; h < (valid1 ? 2 : 1); ++h)
+            for (int i = t; i < N; i += kThreads) {
+                const float2 v = cell(i >> 6, i & 63);
+                p.planes[(size_t)(w0 + h) * N + i] = 0.25f * (h ? v.y : v.x);
+            }
 
     // ---- find_peaks on both planes at once: thread = (column, 16-row
-    // block); rows roll through registers, the horizontal neighbours come
-    // from the neighbouring lanes (the two edge lanes read theirs)
-    Top2 s0, s1;
-    s0.init();
-    s1.init();
+    // block); its column rolls through registers
+    Top2 s[2];
+    s[0].init();
+    s[1].init();
     {
         const int xs = t & 63, yb = (t >> 6) * 16;
-        const bool col_ok = xs >= SX0 && xs < SX1;
-        auto cell = [&](int ys, int x) -> float2 {   // swapped-plane values of both planes
-            return T1[at((ys + W / 2) & (W - 1), (x + W / 2) & (W - 1))];
-        };
-        float2 up = cell(yb - 1, xs), cc = cell(yb, xs);
-        for (int ys = yb; ys < yb + 16; ++ys) {
-            const float2 dn = cell(ys + 1, xs);
-            float2 lf = make_float2(__shfl_up_sync(0xffffffffu, cc.x, 1), __shfl_up_sync(0xffffffffu, cc.y, 1));
-            float2 rt = make_float2(__shfl_down_sync(0xffffffffu, cc.x, 1), __shfl_down_sync(0xffffffffu, cc.y, 1));
-            if (lane == 0) lf = cell(ys, xs - 1);
-            if (lane == 31) rt = cell(ys, xs + 1);
-            if (col_ok && ys >= SY0 && ys < SY1) {
-                s0.add(cc.x, fmaxf(fmaxf(up.x, dn.x), fmaxf(lf.x, rt.x)), dlt, ys * W + xs);
-                s1.add(cc.y, fmaxf(fmaxf(up.y, dn.y), fmaxf(lf.y, rt.y)), dlt, ys * W + xs);
+        if (yb + 16 > SY0 && yb < SY1) {   // warp-uniform
+            const float2* row = T + ((yb + W / 2) & (W - 1));
+            const float2* cc0 = row + ((xs + W / 2) & (W - 1)) * LD;
+            const float2* lf0 = row + ((xs + W / 2 - 1) & (W - 1)) * LD;
+            const float2* rt0 = row + ((xs + W / 2 + 1) & (W - 1)) * LD;
+            float2 up = cell(yb - 1, xs), cc = cc0[0];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const float2 dn = i < 15 ? cc0[i + 1] : cell(yb + 16, xs);
+                const float2 lf = lf0[i], rt = rt0[i];
+                const int ys = yb + i;
+                if (ys >= SY0 && ys < SY1) {
+                    s[0].add(cc.x, max4(up.x, dn.x, lf.x, rt.x), dlt, i);
+                    s[1].add(cc.y, max4(up.y, dn.y, lf.y, rt.y), dlt, i);
+                }
+                up = cc;
+                cc = dn;
             }
-            up = cc;
-            cc = dn;
+            s[0].key = (yb + s[0].key) * W + xs;   // unused where nothing was found
+            s[1].key = (yb + s[1].key) * W + xs;
+            if (xs < SX0 || xs >= SX1) {
+                s[0].init();
+                s[1].init();
+            }
         }
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        s[0].merge(o);
+        s[1].merge(o);
+    }
+    if (lane < 2) s_top[lane][warp] = lane ? s[1] : s[0];
+    __syncthreads();
 
-    for (int h = 0; h < 2; ++h) {
-        const int w = h ? w1 : w0;
-        const bool valid = h ? valid1 : true;
-        const float ped = sped[h];
-        auto val = [&](int ys, int xs) -> float {   // swapped-plane value
-            const float2 v = T1[at((ys + W / 2) & (W - 1), (xs + W / 2) & (W - 1))];
+    // ---- window h: warp h reduces, fits and writes
+    if (warp < 2 && (warp == 0 || valid1)) {
+        const int h = warp, w = w0 + h;
+        Top2 g = s_top[h][lane & (kWarps - 1)];
+        g.merge(4);
+        g.merge(2);
+        g.merge(1);
+        const float ped = s_ped[h];
+        auto val = [&](int ys, int xs) -> float {
+            const float2 v = cell(ys, xs);
             return h ? v.y : v.x;
         };
-        if (PLANES && valid)
-            for (int i = t; i < N; i += kThreads)
-                p.planes[(size_t)w * N + i] = 0.25f * val(i >> 6, i & 63);
-
-        float t0 = h ? s1.t0 : s0.t0, t1 = h ? s1.t1 : s0.t1, umax = h ? s1.umax : s0.umax;
-        int key = h ? s1.key : s0.key;
-        // warp reduction (ties to the lowest row-major index)
-        for (int o = 16; o > 0; o >>= 1) {
-            const float o0 = __shfl_xor_sync(0xffffffffu, t0, o);
-            const float o1 = __shfl_xor_sync(0xffffffffu, t1, o);
-            const int ok = __shfl_xor_sync(0xffffffffu, key, o);
-            const bool take = (o0 > t0) || (o0 == t0 && ok < key);
-            const float n1 = take ? fmaxf(t0, o1) : fmaxf(t1, o0);
-            t0 = take ? o0 : t0;
-            key = take ? ok : key;
-            t1 = n1;
-            umax = fmaxf(umax, __shfl_xor_sync(0xffffffffu, umax, o));
-        }
-        if (lane == 0) { rv0[wp] = t0; rv1[wp] = t1; rk[wp] = key; ru[wp] = umax; }
-        __syncthreads();
-        if (t == 0) {
-            s_slot[h] = -1;
-            float g0 = kNegInf64, g1 = kNegInf64, gu = kNegInf64;
-            int gk = 0x7fffffff;
-            for (int i = 0; i < kWarps; ++i) {
-                const bool take = (rv0[i] > g0) || (rv0[i] == g0 && rk[i] < gk);
-                const float n1 = take ? fmaxf(g0, rv1[i]) : fmaxf(g1, rv0[i]);
-                if (take) { g0 = rv0[i]; gk = rk[i]; }
-                g1 = n1;
-                gu = fmaxf(gu, ru[i]);
+        const bool has2 = g.t1 > kNegInf64;
+        const int px = has2 ? g.key % W : W / 2, py = has2 ? g.key / W : W / 2;
+        const float vc = val(py, px), vl = val(py, px - 1), vr = val(py, px + 1);
+        const float vu = val(py - 1, px), vd = val(py + 1, px);
+        // the six logarithms on six lanes: ln(L/R), ln(L/C), ln(R/C) and
+        // ln(U/D), ln(U/C), ln(D/C), each as log1p((num - den) / (den + ped))
+        const int q = lane < 6 ? lane : 0;
+        const float an = q == 0 || q == 1 ? vl : q == 2 ? vr : q == 3 || q == 4 ? vu : vd;
+        const float ad = q == 0 ? vr : q == 3 ? vd : vc;
+        const float lg = log1pf((an - ad) / (ad + ped));
+        const float lxr = __shfl_sync(0xffffffffu, lg, 0), lyd = __shfl_sync(0xffffffffu, lg, 3);
+        const float denx = __shfl_sync(0xffffffffu, lg, 1) + __shfl_sync(0xffffffffu, lg, 2);
+        const float deny = __shfl_sync(0xffffffffu, lg, 4) + __shfl_sync(0xffffffffu, lg, 5);
+        int slot = -1;
+        if (lane == 0) {
+            int bx, by, ox, oy;
+            window_origin(p, w, bx, by);
+            b_offset(p, W, bx, by, ox, oy);
+            opiv_vector out{ 0.f, 0.f, 0.f, 0.f, 0.f };
+            int32_t code = -1;
+            bool certain;
+            if (!has2) {
+                certain = !(g.umax > kNegInf64);
+            } else {
+                const float C = vc + ped, L = vl + ped, R = vr + ped, U = vu + ped, D = vd + ped;
+                const float nan = __int_as_float(0x7fffffff);
+                const bool okx = L > 0.f && C > 0.f && R > 0.f;
+                const bool oky = U > 0.f && C > 0.f && D > 0.f;
+                const float fx = okx ? lxr / (2.f * denx) : nan;
+                const float fy = oky ? lyd / (2.f * deny) : nan;
+                const float mx = fminf(fminf(L, R), C), my = fminf(fminf(U, D), C);
+                const float ex = okx ? (denx == 0.f ? 3.4e38f
+                                        : dlt * (1.f + 4.f * fabsf(fx)) / (mx * 2.f * fabsf(denx)))
+                                     : (mx < -dlt ? 0.f : 3.4e38f);
+                const float ey = oky ? (deny == 0.f ? 3.4e38f
+                                        : dlt * (1.f + 4.f * fabsf(fy)) / (my * 2.f * fabsf(deny)))
+                                     : (my < -dlt ? 0.f : 3.4e38f);
+                const float p0 = g.t0 + ped, p1 = g.t1 + ped;
+                const float sn_err = 0.5f * dlt * (1.f / fabsf(p0) + 1.f / fabsf(p1));
+                certain = (g.umax < g.t1 - 2.f * dlt) && (g.t0 - g.t1 > dlt) && (fabsf(p1) > dlt) &&
+                          (ex < kFitTol) && (ey < kFitTol) &&
+                          (p1 <= 0.f || sn_err < kSnTol * (1.f + p0 / p1));
+                out.x = (float)(bx + W / 2);
+                out.y = (float)(p.img_h - (by + W / 2));
+                out.u = (float)(W / 2 - px - ox) - fx;
+                out.v = (float)(W / 2 - py - oy) - fy;
+                out.sn = (p1 > 0.f) ? p0 / p1 : 0.f;
+                code = g.key;
             }
-            if (valid) {
-                opiv_vector out{ 0.f, 0.f, 0.f, 0.f, 0.f };
-                int32_t code = -1;
-                bool certain;
-                if (!(g1 > kNegInf64)) {
-                    certain = !(gu > kNegInf64);
-                } else {
-                    const int px = gk % W, py = gk / W;
-                    const float vc = val(py, px), vl = val(py, px - 1), vr = val(py, px + 1);
-                    const float vu = val(py - 1, px), vd = val(py + 1, px);
-                    const float C = vc + ped, L = vl + ped, R = vr + ped, U = vu + ped, D = vd + ped;
-                    const float nan = __int_as_float(0x7fffffff);
-                    const bool okx = L > 0.f && C > 0.f && R > 0.f;
-                    const bool oky = U > 0.f && C > 0.f && D > 0.f;
-                    const float denx = log1pf((vl - vc) / C) + log1pf((vr - vc) / C);
-                    const float deny = log1pf((vu - vc) / C) + log1pf((vd - vc) / C);
-                    const float fx = okx ? log1pf((vl - vr) / R) / (2.f * denx) : nan;
-                    const float fy = oky ? log1pf((vu - vd) / D) / (2.f * deny) : nan;
-                    const float mx = fminf(fminf(L, R), C), my = fminf(fminf(U, D), C);
-                    const float ex = okx ? (denx == 0.f ? 3.4e38f
-                                            : dlt * (1.f + 4.f * fabsf(fx)) / (mx * 2.f * fabsf(denx)))
-                                         : (mx < -dlt ? 0.f : 3.4e38f);
-                    const float ey = oky ? (deny == 0.f ? 3.4e38f
-                                            : dlt * (1.f + 4.f * fabsf(fy)) / (my * 2.f * fabsf(deny)))
-                                         : (my < -dlt ? 0.f : 3.4e38f);
-                    const float p0 = g0 + ped, p1 = g1 + ped;
-                    const float sn_err = 0.5f * dlt * (1.f / fabsf(p0) + 1.f / fabsf(p1));
-                    certain = (gu < g1 - 2.f * dlt) && (g0 - g1 > dlt) && (fabsf(p1) > dlt) &&
-                              (ex < kFitTol) && (ey < kFitTol) &&
-                              (p1 <= 0.f || sn_err < kSnTol * (1.f + p0 / p1));
-                    const int bx = h ? bx1 : bx0, by = h ? by1 : by0;
-                    out.x = (float)(bx + W / 2);
-                    out.y = (float)(p.img_h - (by + W / 2));
-                    out.u = (float)(W / 2 - px - (h ? ox1 : ox0)) - fx;
-                    out.v = (float)(W / 2 - py - (h ? oy1 : oy0)) - fy;
-                    out.sn = (p1 > 0.f) ? p0 / p1 : 0.f;
-                    code = gk;
-                }
-                p.out_vec[w] = out;
-                if (p.out_peak) p.out_peak[w] = code;
-                if (p.out_disp) {
-                    const int ox = h ? ox1 : ox0, oy = h ? oy1 : oy0;
-                    p.out_disp[w] = code >= 0 ? pack_disp(gk % W - W / 2 + ox, gk / W - W / 2 + oy)
-                                              : pack_disp(ox, oy);
-                }
-                if (!certain && p.flag_list) {
-                    const unsigned int at = atomicAdd(p.flag_count, 1u);
-                    p.flag_list[at] = (int32_t)w + p.flag_base;
-                    if (at < (unsigned int)p.flag_cap) s_slot[h] = (int)at;
-                }
+            p.out_vec[w] = out;
+            if (p.out_peak) p.out_peak[w] = code;
+            if (p.out_disp)
+                p.out_disp[w] = has2 ? pack_disp(px - W / 2 + ox, py - W / 2 + oy) : pack_disp(ox, oy);
+            if (!certain && p.flag_list) {
+                const unsigned int at = atomicAdd(p.flag_count, 1u);
+                p.flag_list[at] = (int32_t)w + p.flag_base;
+                if (at < (unsigned int)p.flag_cap) slot = (int)at;
             }
         }
-        __syncthreads();
-    }
-    // flagged windows hand their planes on
-    if (!PLANES && (s_slot[0] & s_slot[1]) >= 0) {
-#pragma unroll 1
-        for (int h = 0; h < 2; ++h) {
-            if (s_slot[h] < 0) continue;
-            float* rec = p.flag_planes + (size_t)s_slot[h] * flag_record_floats(W);
-            for (int i = t; i < N; i += kThreads) {
-                const float2 v = T1[at(((i >> 6) + W / 2) & (W - 1), (i + W / 2) & (W - 1))];
-                rec[i] = h ? v.y : v.x;
-            }
-            if (t == 0) rec[N] = dlt;
+        // a flagged window hands its plane on
+        if (!PLANES) slot = __shfl_sync(0xffffffffu, slot, 0);
+        if (!PLANES && slot >= 0) {
+            float* rec = p.flag_planes + (size_t)slot * flag_record_floats(W);
+            for (int i = lane; i < N; i += 32) rec[i] = val(i >> 6, i & 63);
+            if (lane == 0) rec[N] = dlt;
         }
-        __syncthreads();   // T1 and the slots are the next task's
     }
 }
 
 template <int MODE, bool LIMIT, typename PixT, bool PLANES>
-__global__ void __launch_bounds__(kThreads, 3)
+__global__ void __launch_bounds__(kThreads, kCtasPerSm)
 piv_w64_kernel(const PivParams p)
 {
     w64_task<MODE, LIMIT, PixT, PLANES>(p, (int)blockIdx.x);
@@ -460,7 +643,7 @@ __device__ __forceinline__ const PivParams& cta_item(const PivQueue& q, int j, P
 }
 
 template <int MODE, bool LIMIT, typename PixT>
-__global__ void __launch_bounds__(kThreads, 3)
+__global__ void __launch_bounds__(kThreads, kCtasPerSm)
 piv_w64_queue_kernel(const __grid_constant__ PivQueue q)
 {
     __shared__ unsigned int s_t0;
@@ -480,7 +663,7 @@ piv_w64_queue_kernel(const __grid_constant__ PivQueue q)
 #pragma unroll 1
         for (int t = (int)t0; t < t1; ++t) {
             const int j = __ldg(q.task_item + t);
-            // the task ends with a barrier: the previous descriptor is no longer read
+            __syncthreads();   // the previous task's tile and descriptor are no longer read
             const PivParams& p = cta_item(q, j, reinterpret_cast<PivParams*>(s_item));
             w64_task<MODE, LIMIT, PixT, false>(p, t - q.first_task[j]);
         }
@@ -490,7 +673,7 @@ piv_w64_queue_kernel(const __grid_constant__ PivQueue q)
 template <int MODE, bool LIMIT, typename PixT, bool PLANES>
 cudaError_t launch_t(const PivParams& p, cudaStream_t s)
 {
-    const size_t smem = sizeof(float2) * 2 * W * LD;
+    const size_t smem = sizeof(float2) * W * LD;
     static std::atomic<uint64_t> attr_done{ 0 };   // one bit per device
     int dev = 0;
     cudaGetDevice(&dev);
@@ -522,7 +705,7 @@ cudaError_t launch_dt(const PivParams& p, int dtype, bool planes, cudaStream_t s
 // The same work list dispatched by the hardware: CTA b runs task b, no
 // persistent loop.
 template <int MODE, bool LIMIT, typename PixT>
-__global__ void __launch_bounds__(kThreads, 3)
+__global__ void __launch_bounds__(kThreads, kCtasPerSm)
 piv_w64_list_kernel(const __grid_constant__ PivQueue q)
 {
     __shared__ __align__(16) unsigned char s_item[sizeof(PivParams)];
@@ -537,7 +720,7 @@ piv_w64_list_kernel(const __grid_constant__ PivQueue q)
 template <int MODE, bool LIMIT, typename PixT>
 cudaError_t queue_t(const PivQueue& q, int blocks, int* max_ctas, cudaStream_t s)
 {
-    const size_t smem = sizeof(float2) * 2 * W * LD;
+    const size_t smem = sizeof(float2) * W * LD;
     auto kern = piv_w64_queue_kernel<MODE, LIMIT, PixT>;
     auto list = piv_w64_list_kernel<MODE, LIMIT, PixT>;
     static std::atomic<uint64_t> attr_done{ 0 };   // one bit per device
