@@ -183,6 +183,7 @@ struct opiv_plan {
     void* d_fa = nullptr;               // frames for the host-buffer calls
     void* d_fb = nullptr;
     size_t d_pitch = 0;
+    unsigned char* d_scratch = nullptr; // one allocation: d_vec .. d_tw
     opiv_vector* d_vec = nullptr;
     int32_t* d_peak = nullptr;
     unsigned int* d_flag_count = nullptr;
@@ -238,12 +239,7 @@ void plan_free(opiv_plan* p)
     if (p->stream) cudaStreamSynchronize(p->stream);
     cudaFree(p->d_fa);
     cudaFree(p->d_fb);
-    cudaFree(p->d_vec);
-    cudaFree(p->d_peak);
-    cudaFree(p->d_flag_count);
-    cudaFree(p->d_flag_list);
-    cudaFree(p->d_flag_planes);
-    cudaFree(p->d_tw);
+    cudaFree(p->d_scratch);
     cudaFree(p->d_disp);
     cudaFree(p->d_tc);
     cudaFree(p->d_status);
@@ -502,19 +498,25 @@ int plan_create(opiv_plan** out, uint32_t img_w, uint32_t img_h, int dtype, uint
     if ((e = cudaSetDevice(device)) != cudaSuccess) return done(cuda_fail(e, "cudaSetDevice"));
     if ((e = cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking)) != cudaSuccess)
         return done(cuda_fail(e, "cudaStreamCreate"));
-    if ((e = cudaMalloc(&p->d_vec, sizeof(opiv_vector) * p->n_win)) != cudaSuccess)
-        return done(cuda_fail(e, "cudaMalloc(vectors)"));
-    if ((e = cudaMalloc(&p->d_peak, sizeof(int32_t) * p->n_win)) != cudaSuccess)
-        return done(cuda_fail(e, "cudaMalloc(peaks)"));
-    if ((e = cudaMalloc(&p->d_flag_count, sizeof(unsigned int))) != cudaSuccess)
-        return done(cuda_fail(e, "cudaMalloc(flag count)"));
-    if ((e = cudaMalloc(&p->d_flag_list, sizeof(int32_t) * p->n_win)) != cudaSuccess)
-        return done(cuda_fail(e, "cudaMalloc(flag list)"));
-    if (!tc_only) {   // passes of the tensor-core path flag nothing
-        p->flag_cap = flag_capacity(p->n_win, ia);
-        if ((e = cudaMalloc(&p->d_flag_planes, flag_plane_bytes(p->flag_cap, ia))) != cudaSuccess)
-            return done(cuda_fail(e, "cudaMalloc(flagged planes)"));
-    }
+    // one allocation for the plan's outputs and scratch (each costs about as
+    // much as all of them together)
+    if (!tc_only) p->flag_cap = flag_capacity(p->n_win, ia);   // the tensor-core path flags nothing
+    size_t bytes = 0;
+    auto part = [&](size_t size) {
+        const size_t at = bytes;
+        bytes += (size + 255) / 256 * 256;
+        return at;
+    };
+    const size_t at_vec = part(sizeof(opiv_vector) * p->n_win), at_peak = part(sizeof(int32_t) * p->n_win);
+    const size_t at_count = part(sizeof(unsigned int)), at_list = part(sizeof(int32_t) * p->n_win);
+    const size_t at_planes = part(flag_plane_bytes(p->flag_cap, ia)), at_tw = part(sizeof(double2) * 2 * ia);
+    if ((e = cudaMalloc(&p->d_scratch, bytes)) != cudaSuccess) return done(cuda_fail(e, "cudaMalloc(plan scratch)"));
+    p->d_vec = reinterpret_cast<opiv_vector*>(p->d_scratch + at_vec);
+    p->d_peak = reinterpret_cast<int32_t*>(p->d_scratch + at_peak);
+    p->d_flag_count = reinterpret_cast<unsigned int*>(p->d_scratch + at_count);
+    p->d_flag_list = reinterpret_cast<int32_t*>(p->d_scratch + at_list);
+    p->d_flag_planes = reinterpret_cast<float*>(p->d_scratch + at_planes);
+    p->d_tw = reinterpret_cast<double2*>(p->d_scratch + at_tw);
     if ((e = cudaMemset(p->d_flag_count, 0, sizeof(unsigned int))) != cudaSuccess)
         return done(cuda_fail(e, "cudaMemset"));
     if ((e = cudaMallocHost(&p->h_flag_count, sizeof(unsigned int))) != cudaSuccess)
@@ -523,8 +525,6 @@ int plan_create(opiv_plan** out, uint32_t img_w, uint32_t img_h, int dtype, uint
     if (is_pow2(ia)) {   // the exact kernel's twiddles (FFT path)
         std::vector<double2> tw = reference_twiddles(ia, -1), tr = reference_twiddles(ia, +1);
         tw.insert(tw.end(), tr.begin(), tr.end());
-        if ((e = cudaMalloc(&p->d_tw, sizeof(double2) * tw.size())) != cudaSuccess)
-            return done(cuda_fail(e, "cudaMalloc(twiddles)"));
         if ((e = cudaMemcpy(p->d_tw, tw.data(), sizeof(double2) * tw.size(), cudaMemcpyHostToDevice)) !=
             cudaSuccess)
             return done(cuda_fail(e, "cudaMemcpy(twiddles)"));
