@@ -93,60 +93,49 @@ constexpr TwiddleTable make_twiddles()
 static __constant__ TwiddleTable c_tw = make_twiddles();
 
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
-
-// z * exp(-+2*pi*i*k/N); INV selects the + sign.
-template <int N, bool INV>
-__device__ __forceinline__ float2 twiddle(float2 z, int k)
+// Packed FP32 pairs (one instruction for both components; each rounds as the
+// scalar one does).
+__device__ __forceinline__ float2 add2(float2 a, float2 b)
 {
-    k &= (N - 1);
-    if (k == 0) return z;
-    if (4 * k == N) return INV ? make_float2(-z.y, z.x) : make_float2(z.y, -z.x);
-    if (2 * k == N) return make_float2(-z.x, -z.y);
-    if (4 * k == 3 * N) return INV ? make_float2(z.y, -z.x) : make_float2(-z.y, z.x);
-    const float wr = c_tw.re[k * (kTwMax / N)];
-    const float wi = INV ? -c_tw.im[k * (kTwMax / N)] : c_tw.im[k * (kTwMax / N)];
-    return make_float2(z.x * wr - z.y * wi, z.x * wi + z.y * wr);
+    float2 d;
+    asm("{ .reg .b64 x, y; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; add.rn.f32x2 x, x, y; mov.b64 {%0, %1}, x; }"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+__device__ __forceinline__ float2 sub2(float2 a, float2 b)
+{
+    float2 d;
+    asm("{ .reg .b64 x, y; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; sub.rn.f32x2 x, x, y; mov.b64 {%0, %1}, x; }"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
 }
 
-// Decimation in frequency: natural-order input, bit-reversed output
-// (v[i] holds X[bitrev(i)]).
-template <int N, bool INV>
-__device__ __forceinline__ void fft_dif(float2 (&v)[N])
+__device__ __forceinline__ float2 mul2(float2 a, float2 b)
 {
-#pragma unroll
-    for (int half = N / 2; half >= 1; half >>= 1) {
-#pragma unroll
-        for (int base = 0; base < N; base += 2 * half) {
-#pragma unroll
-            for (int j = 0; j < half; ++j) {
-                const float2 a = v[base + j], b = v[base + j + half];
-                v[base + j] = cadd(a, b);
-                v[base + j + half] = twiddle<N, INV>(csub(a, b), j * (N / (2 * half)));
-            }
-        }
-    }
+    float2 d;
+    asm("{ .reg .b64 x, y; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; mul.rn.f32x2 x, x, y; mov.b64 {%0, %1}, x; }"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
+{
+    float2 d;
+    asm("{ .reg .b64 x, y, z; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; mov.b64 z, {%6, %7}; "
+        "fma.rn.f32x2 x, x, y, z; mov.b64 {%0, %1}, x; }"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
 }
 
-// Decimation in time: bit-reversed input (v[i] holds x[bitrev(i)]),
-// natural-order output.
-template <int N, bool INV>
-__device__ __forceinline__ void fft_dit(float2 (&v)[N])
+// 4 conj(P) = ( 2 Im(Z Zm), |Z|^2 - |Zm|^2 ) of a bin of Z = FFT(a + i b) and
+// its mirror Zm = Z[-k], P = B conj(A).  With s = Z + Zm and t = Z - Zm,
+// 2 A = (s.x, t.y) and 2 B = (s.y, -t.x): formed from those, the rounding is
+// that of A's and B's own product (squares of Z would round in units of
+// |A|^2 + |B|^2, and one product serves both k and -k, so the two bins'
+// roundings do not average out).
+__device__ __forceinline__ float2 four_conj_p(float2 z, float2 m)
 {
-#pragma unroll
-    for (int half = 1; half < N; half <<= 1) {
-#pragma unroll
-        for (int base = 0; base < N; base += 2 * half) {
-#pragma unroll
-            for (int j = 0; j < half; ++j) {
-                const float2 a = v[base + j];
-                const float2 b = twiddle<N, INV>(v[base + j + half], j * (N / (2 * half)));
-                v[base + j] = cadd(a, b);
-                v[base + j + half] = csub(a, b);
-            }
-        }
-    }
+    const float2 s = add2(z, m), t = sub2(z, m);
+    return make_float2(fmaf(s.x, s.y, -(t.x * t.y)), fmaf(s.x, t.x, s.y * t.y));
 }
 
 // ---------------------------------------------------------------------------
@@ -155,7 +144,8 @@ __device__ __forceinline__ void fft_dit(float2 (&v)[N])
 // c = b + i t b and 4 FMAs for a +- wx*c: 6 instructions per twiddled
 // butterfly instead of 8.  The factor with the larger magnitude is pulled
 // out (wx when |wx| >= |wy|, else wy with w*b = wy * ((wx/wy) b + i b)), which
-// keeps the ratio within [-1, 1].  Tables are evaluated at compile time.
+// keeps the ratio within [-1, 1].  The last four are two packed ones.  Tables
+// are evaluated at compile time.
 struct FmaTwiddles {
     float m[kTwMax];      // pulled-out factor: wx or wy of exp(-2 pi i k / 64)
     float r[kTwMax];      // ratio: wy / wx or wx / wy
@@ -193,14 +183,14 @@ __device__ __forceinline__ void bfly_dit(float2& a, float2& b, int k)
     k &= (N - 1);
     if (k == 0) {
         const float2 t = b;
-        b = csub(a, t);
-        a = cadd(a, t);
+        b = sub2(a, t);
+        a = add2(a, t);
         return;
     }
     if (4 * k == N) {   // w = -i (forward) or i (inverse)
         const float2 wb = INV ? make_float2(-b.y, b.x) : make_float2(b.y, -b.x);
-        b = csub(a, wb);
-        a = cadd(a, wb);
+        b = make_float2(a.x - wb.x, a.y - wb.y);
+        a = make_float2(a.x + wb.x, a.y + wb.y);
         return;
     }
     const int q = k * (kTwMax / N);
@@ -212,8 +202,8 @@ __device__ __forceinline__ void bfly_dit(float2& a, float2& b, int k)
     } else {                // w b = wy (s bx - by, s by + bx), s = wx / wy
         c = make_float2(fmaf(r, b.x, -b.y), fmaf(r, b.y, b.x));
     }
-    b = make_float2(fmaf(-m, c.x, a.x), fmaf(-m, c.y, a.y));
-    a = make_float2(fmaf(m, c.x, a.x), fmaf(m, c.y, a.y));
+    b = fma2(make_float2(-m, -m), c, a);
+    a = fma2(make_float2(m, m), c, a);
 }
 
 // Decimation in time, FMA form: bit-reversed input (v[i] holds

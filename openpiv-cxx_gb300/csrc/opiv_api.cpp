@@ -114,13 +114,14 @@ std::vector<double2> reference_twiddles(uint32_t n, int dir)
 int exact_blocks(int device) { return 2 * device_sm_count(device); }
 int exact_all_blocks(int device) { return 8 * device_sm_count(device); }
 
-// Flagged windows whose planes a pass keeps for refine_window: particle
-// images flag up to one window in a hundred; beyond this room (or 4 MiB)
-// the exact kernel decides them from the frames alone.
+// Flagged windows whose planes a pass keeps for refine_window: one in eight
+// of 16 px windows (REAL mode with the limited search flags up to 13 %, other
+// fields up to 4 %), one in 32 of larger ones (below 1 %), 16 MiB at most; the
+// exact kernel decides those beyond from the frames alone.
 int32_t flag_capacity(int64_t n_win, uint32_t ia)
 {
-    const int64_t room = (int64_t)(4u << 20) / (int64_t)(sizeof(float) * flag_record_floats((int)ia));
-    return (int32_t)std::min({ n_win, 64 + n_win / 32, room });
+    const int64_t room = (int64_t)(16u << 20) / (int64_t)(sizeof(float) * flag_record_floats((int)ia));
+    return (int32_t)std::min({ n_win, 64 + n_win / (ia <= 16 ? 8 : 32), room });
 }
 size_t flag_plane_bytes(int32_t cap, uint32_t ia)
 {

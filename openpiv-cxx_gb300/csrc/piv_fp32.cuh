@@ -13,7 +13,9 @@
 //   the two-for-one unpack and the product in one step: with Zm = Z[-k]
 //   (fetched from the mirror lane by a shuffle),
 //       P = B conj(A) = ( Im(Z Zm) / 2 , (|Zm|^2 - |Z|^2) / 4 ),
-//   which is FFT(b) conj(FFT(a)) of fft.h:188-227; REAL mode leaves the
+//   formed from the sums and differences Z +- Zm, which are A's and B's
+//   components, and once per pair of bins k, -k (P is Hermitian);
+//   this is FFT(b) conj(FFT(a)) of fft.h:188-227; REAL mode leaves the
 //   reference's unpacked set only (fft.h:166-183: spectrum row 0, row W/2
 //   and column 0 stay zero), done by zeroing those Z rows / the Z column;
 //   the products of the pair are packed as Q = conj(P1) + i conj(P2): both
@@ -61,22 +63,27 @@ constexpr int kWarps = 4;   // warps per CTA
 // those tolerances (the rounding of the final FP32 logarithms, sums and
 // ratio adds ~1e-6 px and ~2e-7 relative on top of the bounds).  At 3e-5 /
 // 3e-6 three times as many 16 px windows went to the exact pass, nearly all
-// of them for the sn bound.
+// of them for the sn bound.  The factor 1 + sn ends at kSnCap: a few windows
+// of sn in the tens, whose second peak is little more than rounding, carried
+// nearly all of a field's sn error (2048 x 1536 field of 16 px windows: 1e-6 of
+// its norm, 1e-7 with the cap, 139 windows flagged where 78 were; REAL mode
+// with the limited search up to 1.5e-3 and 4e-8).
 constexpr float kFitTol = 6e-5f;
 constexpr float kSnTol = 6e-6f;
+constexpr float kSnCap = 4.f;
 #define kNegInf (-__int_as_float(0x7f800000))
 constexpr float kTwo23 = 8388608.0f;
 
 // ---- pixel loading -----------------------------------------------------------
 // Exact widening of 8/16-bit pixels: bits 0x4B000000 | u are the float
-// 2^23 + u (u < 2^23); subtracting 2^23 is exact.
-__device__ __forceinline__ float u16_lo(uint32_t w) { return __int_as_float(__byte_perm(w, 0x4B00, 0x5410)) - kTwo23; }
-__device__ __forceinline__ float u16_hi(uint32_t w) { return __int_as_float(__byte_perm(w, 0x4B00, 0x5432)) - kTwo23; }
+// 2^23 + u (u < 2^23); subtracting 2^23 (from both frames' pixels at once,
+// when both rows are in) is exact.
+__device__ __forceinline__ float u16_lo(uint32_t w) { return __int_as_float(__byte_perm(w, 0x4B00, 0x5410)); }
+__device__ __forceinline__ float u16_hi(uint32_t w) { return __int_as_float(__byte_perm(w, 0x4B00, 0x5432)); }
 template <int K>
-__device__ __forceinline__ float u8_k(uint32_t w) { return __int_as_float(__byte_perm(w, 0x4B00, 0x5440 | K)) - kTwo23; }
+__device__ __forceinline__ float u8_k(uint32_t w) { return __int_as_float(__byte_perm(w, 0x4B00, 0x5440 | K)); }
 
-// W consecutive pixels starting at `ptr` into the x (A) or y (B) components
-// of v.  VEC: the row start is 16-byte aligned.
+// Component x (frame A) or y (frame B) of an element.
 template <bool B>
 __device__ __forceinline__ void put(float2& z, float f)
 {
@@ -86,10 +93,10 @@ __device__ __forceinline__ void put(float2& z, float f)
 
 // Pixel x goes to register bitrev(x): the row transform takes bit-reversed
 // input.
-template <int W, bool B, typename PixT, bool VEC>
+template <int W, bool B, typename PixT>
 __device__ __forceinline__ void load_row(const PixT* ptr, float2 (&v)[W])
 {
-    if (VEC && sizeof(PixT) == 2) {
+    if (sizeof(PixT) == 2) {
         const uint4* q = reinterpret_cast<const uint4*>(ptr);
 #pragma unroll
         for (int k = 0; k < W / 8; ++k) {
@@ -99,7 +106,7 @@ __device__ __forceinline__ void load_row(const PixT* ptr, float2 (&v)[W])
             put<B>(v[bitrev<W>(8 * k + 4)], u16_lo(r.z)); put<B>(v[bitrev<W>(8 * k + 5)], u16_hi(r.z));
             put<B>(v[bitrev<W>(8 * k + 6)], u16_lo(r.w)); put<B>(v[bitrev<W>(8 * k + 7)], u16_hi(r.w));
         }
-    } else if (VEC && sizeof(PixT) == 1) {
+    } else if (sizeof(PixT) == 1) {
         const uint4* q = reinterpret_cast<const uint4*>(ptr);
 #pragma unroll
         for (int k = 0; k < W / 16; ++k) {
@@ -113,7 +120,7 @@ __device__ __forceinline__ void load_row(const PixT* ptr, float2 (&v)[W])
                 put<B>(v[bitrev<W>(16 * k + 4 * j + 3)], u8_k<3>(w4[j]));
             }
         }
-    } else if (VEC && sizeof(PixT) == 4) {
+    } else if (sizeof(PixT) == 4) {
         const float4* q = reinterpret_cast<const float4*>(ptr);
 #pragma unroll
         for (int k = 0; k < W / 4; ++k) {
@@ -121,24 +128,20 @@ __device__ __forceinline__ void load_row(const PixT* ptr, float2 (&v)[W])
             put<B>(v[bitrev<W>(4 * k + 0)], r.x); put<B>(v[bitrev<W>(4 * k + 1)], r.y);
             put<B>(v[bitrev<W>(4 * k + 2)], r.z); put<B>(v[bitrev<W>(4 * k + 3)], r.w);
         }
-    } else {
-#pragma unroll
-        for (int x = 0; x < W; ++x) put<B>(v[bitrev<W>(x)], (float)__ldg(ptr + x));
     }
 }
 
-// A row that starts anywhere (B windows shifted by a previous pass's
-// displacement): the 16-byte blocks covering it are loaded whole and the
-// row is shifted out of them by the start's offset inside its block (a
-// word select, then a byte permute).  The blocks read hold at least one
-// pixel of the row each, so they lie inside the frame's allocation.
+// A row that starts anywhere (an unaligned grid or pitch, B windows shifted
+// by a previous pass's displacement): the 16-byte blocks covering it are
+// loaded whole and the row is shifted out of them by the start's offset
+// inside its block (a word select, then a byte permute).  The blocks read
+// hold at least one pixel of the row each, so they lie inside the frame's
+// allocation.  (Element by element a 1531 x 1117 u8 pair of 32 px REAL windows
+// took 77 us; with everything else as here it takes 41.)
 template <int W, bool B, typename PixT>
 __device__ __forceinline__ void load_row_shifted(const PixT* ptr, float2 (&v)[W])
 {
-    if constexpr (sizeof(PixT) > 4) {   // double frames: element loads
-#pragma unroll
-        for (int x = 0; x < W; ++x) put<B>(v[bitrev<W>(x)], (float)__ldg(ptr + x));
-    } else {
+    {
         constexpr int NW = W * (int)sizeof(PixT) / 4;   // 32-bit words of the row
         constexpr int NC = NW / 4;                      // whole blocks of the row
         const uintptr_t a = reinterpret_cast<uintptr_t>(ptr);
@@ -177,6 +180,125 @@ __device__ __forceinline__ void load_row_shifted(const PixT* ptr, float2 (&v)[W]
     }
 }
 
+// 32 px windows of 16-bit frames: a lane that loads its own row makes every
+// 128-bit load touch 32 cache lines, 16 bytes of each, and the L1 is the
+// kernel's busiest unit.  The lanes instead load blocks with neighbouring
+// lanes on neighbouring blocks of a row, put them into the group's tile, and
+// each lane reads its row from there; rows lie an odd number of blocks
+// apart, so the eight lanes of a phase read distinct banks.  A 4096 x 4096
+// pair at step 8 takes 709 us with this and 758 without; rows of 8-bit
+// frames (42.1 against 41.0 us, 1531 x 1117), of float frames (full sectors
+// as it is, and the registers spill) and of 16 px windows (40.5 against
+// 40.4) gain nothing and are loaded by their own lanes.
+template <int W, typename PixT>
+struct row_stage {
+    static constexpr int NC = W * (int)sizeof(PixT) / 16;   // whole blocks of a row
+    static constexpr int LD = (NC + 1) | 1;                 // blocks between rows
+    static constexpr int bytes = 16 * LD * W;
+};
+
+template <int W, bool ALIGNED, typename PixT>
+__device__ __forceinline__ void stage_load(const PixT* corner, size_t pitch, int gl,
+                                           uint4 (&r)[row_stage<W, PixT>::NC + 1])
+{
+    constexpr int NC = row_stage<W, PixT>::NC, PER = ALIGNED ? NC : NC + 1;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const int i = gl + W * k, row = i / PER, c = i % PER;
+        const PixT* ptr = corner + (size_t)row * pitch;
+        if constexpr (ALIGNED) {
+            r[k] = __ldg(reinterpret_cast<const uint4*>(ptr) + c);
+        } else {
+            const uintptr_t a = reinterpret_cast<uintptr_t>(ptr);
+            r[k] = make_uint4(0u, 0u, 0u, 0u);
+            if (c < NC || (a & 15) != 0)   // only a misaligned row reaches into the last block
+                r[k] = __ldg(reinterpret_cast<const uint4*>(a & ~(uintptr_t)15) + c);
+        }
+    }
+}
+
+template <int W, bool ALIGNED, typename PixT>
+__device__ __forceinline__ void stage_store(uint4* tile, int gl, const uint4 (&r)[row_stage<W, PixT>::NC + 1])
+{
+    constexpr int NC = row_stage<W, PixT>::NC, PER = ALIGNED ? NC : NC + 1;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        const int i = gl + W * k;
+        tile[(i / PER) * row_stage<W, PixT>::LD + i % PER] = r[k];
+    }
+}
+
+// The lane's row from the tile into the x (A) or y (B) components of v, at
+// bit-reversed places (the row transform takes bit-reversed input).  `ptr`:
+// the row's start in the frame.
+template <int W, bool B, bool ALIGNED, typename PixT>
+__device__ __forceinline__ void stage_read(const uint4* tile, int gl, const PixT* ptr, float2 (&v)[W])
+{
+    constexpr int NC = row_stage<W, PixT>::NC, NW = 4 * NC;   // 32-bit words of the row
+    uint32_t w[NW + 4];
+#pragma unroll
+    for (int c = 0; c < (ALIGNED ? NC : NC + 1); ++c) {
+        const uint4 r = tile[gl * row_stage<W, PixT>::LD + c];
+        w[4 * c] = r.x; w[4 * c + 1] = r.y; w[4 * c + 2] = r.z; w[4 * c + 3] = r.w;
+    }
+    uint32_t sel = 0x3210u;
+    if constexpr (!ALIGNED) {
+        const int mis = (int)(reinterpret_cast<uintptr_t>(ptr) & 15), ws = mis >> 2;
+        sel += 0x1111u * (uint32_t)(mis & 3);
+#pragma unroll
+        for (int k = 0; k < NW + 2; ++k) w[k] = (ws & 2) ? w[k + 2] : w[k];
+#pragma unroll
+        for (int k = 0; k < NW + 1; ++k) w[k] = (ws & 1) ? w[k + 1] : w[k];
+    }
+#pragma unroll
+    for (int k = 0; k < NW; ++k) {
+        const uint32_t u = ALIGNED ? w[k] : __byte_perm(w[k], w[k + 1], sel);
+        if constexpr (sizeof(PixT) == 2) {
+            put<B>(v[bitrev<W>(2 * k)], u16_lo(u));
+            put<B>(v[bitrev<W>(2 * k + 1)], u16_hi(u));
+        } else if constexpr (sizeof(PixT) == 1) {
+            put<B>(v[bitrev<W>(4 * k + 0)], u8_k<0>(u));
+            put<B>(v[bitrev<W>(4 * k + 1)], u8_k<1>(u));
+            put<B>(v[bitrev<W>(4 * k + 2)], u8_k<2>(u));
+            put<B>(v[bitrev<W>(4 * k + 3)], u8_k<3>(u));
+        } else {
+            put<B>(v[bitrev<W>(k)], __uint_as_float(u));
+        }
+    }
+}
+
+// Both frames' rows of a window (corners ca, cb in their frames): lane = row,
+// registers = columns.  Every lane of the warp calls it; the tile is free
+// again when it returns.
+template <int W, bool AL_A, bool AL_B, typename PixT>
+__device__ __forceinline__ void load_window(const PixT* ca, const PixT* cb, size_t pitch, int gl, uint4* tile,
+                                            float2 (&v)[W])
+{
+    using R = row_stage<W, PixT>;
+    const PixT *pa = ca + (size_t)gl * pitch, *pb = cb + (size_t)gl * pitch;   // the lane's rows
+    if constexpr (W == 32 && sizeof(PixT) == 2) {
+        static_assert(2 * R::bytes <= (int)sizeof(float2) * W * (W + 1), "both frames' rows fit the tile");
+        uint4 ra[R::NC + 1], rb[R::NC + 1];
+        stage_load<W, AL_A, PixT>(ca, pitch, gl, ra);
+        stage_load<W, AL_B, PixT>(cb, pitch, gl, rb);
+        stage_store<W, AL_A, PixT>(tile, gl, ra);
+        stage_store<W, AL_B, PixT>(tile + R::LD * W, gl, rb);
+        __syncwarp();
+        stage_read<W, false, AL_A, PixT>(tile, gl, pa, v);
+        stage_read<W, true, AL_B, PixT>(tile + R::LD * W, gl, pb, v);
+        __syncwarp();
+    } else {
+        if constexpr (AL_A) load_row<W, false, PixT>(pa, v);
+        else load_row_shifted<W, false, PixT>(pa, v);
+        if constexpr (AL_B) load_row<W, true, PixT>(pb, v);
+        else load_row_shifted<W, true, PixT>(pb, v);
+    }
+    if (sizeof(PixT) <= 2) {
+#pragma unroll
+        for (int x = 0; x < W; ++x) v[x] = sub2(v[x], make_float2(kTwo23, kTwo23));
+    }
+}
+
 // Bottom-left corner of window w.  Window indices fit in 32 bits (plans
 // hold at most 2^31 - 1 windows), so the grid position is a 32-bit division.
 __device__ __forceinline__ void window_origin(const PivParams& p, int w, int& bx, int& by)
@@ -198,25 +320,61 @@ __device__ __forceinline__ T group_sum(T x)
     for (int o = W / 2; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o, W);
     return x;
 }
-template <int W>
-__device__ __forceinline__ float group_max(float x)
-{
-#pragma unroll
-    for (int o = W / 2; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o, W));
-    return x;
-}
-
 // W x W tile with rows padded to W + 1 float2: row-wise and column-wise
 // accesses by the W lanes of a group hit distinct banks.
 template <int W>
 __device__ __forceinline__ int tix(int r, int c) { return r * (W + 1) + c; }
-// Hermitian half of a W x W spectrum: columns 0 .. W/2, rows padded.
-template <int W>
-__device__ __forceinline__ int hix(int r, int c) { return r * (W / 2 + 1) + c; }
 
 // shared memory per lane group: transpose tile + half spectrum
 template <int W>
 __host__ __device__ constexpr int group_smem_float2() { return W * (W + 1) + W * (W / 2 + 1); }
+
+// Running top-2 of strict 4-neighbour maxima (find_peaks) plus the largest
+// value whose strict-maximum decision is within dlt of flipping.
+struct Top2 {
+    float t0, t1, umax;
+    int key;
+    __device__ __forceinline__ void init()
+    {
+        t0 = t1 = umax = kNegInf;
+        key = 0;
+    }
+    __device__ __forceinline__ void add(float c, float m, float dlt, int k)
+    {
+        const float dd = m - c;
+        umax = fabsf(dd) <= dlt ? fmaxf(umax, c) : umax;
+        const float v = dd < 0.f ? c : kNegInf;
+        t1 = fmaxf(t1, fminf(t0, v));
+        key = v > t0 ? k : key;
+        t0 = fmaxf(t0, v);
+    }
+    // with another's (ties to the lowest row-major index)
+    __device__ __forceinline__ void merge(const Top2& o)
+    {
+        const bool take = (o.t0 > t0) || (o.t0 == t0 && o.key < key);
+        t1 = fmaxf(fmaxf(t1, o.t1), fminf(t0, o.t0));
+        key = take ? o.key : key;
+        t0 = fmaxf(t0, o.t0);
+        umax = fmaxf(umax, o.umax);
+    }
+    __device__ __forceinline__ Top2 across(int o) const   // the lane o away
+    {
+        Top2 r;
+        r.t0 = __shfl_xor_sync(0xffffffffu, t0, o);
+        r.t1 = __shfl_xor_sync(0xffffffffu, t1, o);
+        r.umax = __shfl_xor_sync(0xffffffffu, umax, o);
+        r.key = __shfl_xor_sync(0xffffffffu, key, o);
+        return r;
+    }
+};
+
+// a three-source max and a max
+__device__ __forceinline__ float max4(float a, float b, float c, float d)
+{
+    float m;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(fmaxf(c, d)));
+    return m;
+}
 
 // Transform stages of a pair, run by one runtime loop around one FFT body.
 enum { kStLoad0 = 0, kStCol0 = 1, kStLoad1 = 2, kStCol1 = 3, kStInvA = 4, kStInvB = 5 };
@@ -242,53 +400,55 @@ __device__ __forceinline__ void fp32_task(const PivParams& p, const int task, fl
     const int first = task * 2 * NG;
     if (first >= (int)p.n_win) return;   // warp-uniform
     float2* S = dyn_smem + (warp * NG + grp) * group_smem_float2<W>();   // transpose tile
-    float2* H = S + W * (W + 1);                                          // first product, half
+    float2* H = S + W * (W + 1);                                          // first product, rows 0 .. W/2
 
     const PixT* fa = reinterpret_cast<const PixT*>(p.fa);
     const PixT* fb = reinterpret_cast<const PixT*>(p.fb);
     const size_t pitch = p.pitch / sizeof(PixT);
 
     float2 v[W];      // the transform being worked on
-    float en0 = 0.f, en1 = 0.f, ped0 = 0.f, ped1 = 0.f;
+    float2 energy = make_float2(0.f, 0.f);
+    float ped0 = 0.f, ped1 = 0.f;
 
 #pragma unroll 1
     for (int st = 0; st < 6; ++st) {
         const int h = (st >= kStLoad1 && st <= kStCol1) ? 1 : 0;
-        const int w = first + h * NG + grp;
-        const bool valid = w < (int)p.n_win;
         // ---------------- before the transform
         if (st == kStLoad0 || st == kStLoad1) {
             // extract + widen: lane = row y, registers = x
-            if (valid) {
-                int bx, by, ox, oy;
-                window_origin(p, w, bx, by);
-                b_offset(p, W, bx, by, ox, oy);
-                const size_t off = (size_t)(by + gl) * pitch + bx;
-                load_row<W, false, PixT, VEC>(fa + off, v);
-                if (p.prev_disp != nullptr)   // shifted B rows need not be aligned
-                    load_row_shifted<W, true, PixT>(fb + (size_t)(by + oy + gl) * pitch + bx + ox, v);
-                else
-                    load_row<W, true, PixT, VEC>(fb + off, v);
-                if (PLANES) {   // exact pedestal for the per-window API (double input)
-                    double sa = 0.0, sb = 0.0;
-#pragma unroll 4
-                    for (int x = 0; x < W; ++x) {
-                        sa += (double)fa[off + x];
-                        sb += (double)fb[off + x];
-                    }
-                    sa = group_sum<W, double>(sa);
-                    sb = group_sum<W, double>(sb);
-                    if (gl == 0) p.peds[w] = (MODE == kModeComplex) ? sa * sb : 0.0;
+            // (a task beyond the last window takes the last one once more and
+            // writes nothing for it: no branch around the loads)
+            const int w = min(first + h * NG + grp, (int)p.n_win - 1);
+            int bx, by, ox, oy;
+            window_origin(p, w, bx, by);
+            b_offset(p, W, bx, by, ox, oy);
+            const PixT* ca = fa + (size_t)by * pitch + bx;
+            const PixT* cb = fb + (size_t)(by + oy) * pitch + bx + ox;
+            if constexpr (PLANES) {   // the per-window API's double frames: element loads
+                double sa = 0.0, sb = 0.0;
+#pragma unroll
+                for (int x = 0; x < W; ++x) {
+                    const double a = (double)__ldg(ca + (size_t)gl * pitch + x);
+                    const double b = (double)__ldg(cb + (size_t)gl * pitch + x);
+                    v[bitrev<W>(x)] = make_float2((float)a, (float)b);
+                    sa += a;
+                    sb += b;
                 }
+                // exact pedestal
+                sa = group_sum<W, double>(sa);
+                sb = group_sum<W, double>(sb);
+                if (gl == 0) p.peds[w] = (MODE == kModeComplex) ? sa * sb : 0.0;
             } else {
-#pragma unroll
-                for (int x = 0; x < W; ++x) v[x] = make_float2(0.f, 0.f);
+                uint4* tile = reinterpret_cast<uint4*>(S);
+                if (!VEC)
+                    load_window<W, false, false, PixT>(ca, cb, pitch, gl, tile, v);
+                else if (p.prev_disp != nullptr)   // shifted B rows need not be aligned
+                    load_window<W, true, false, PixT>(ca, cb, pitch, gl, tile, v);
+                else
+                    load_window<W, true, true, PixT>(ca, cb, pitch, gl, tile, v);
             }
-            float e = 0.f;
 #pragma unroll
-            for (int x = 0; x < W; ++x) e = fmaf(v[x].x, v[x].x, fmaf(v[x].y, v[x].y, e));
-            e = group_sum<W, float>(e);
-            if (h == 0) en0 = e; else en1 = e;
+            for (int x = 0; x < W; ++x) energy = fma2(v[x], v[x], energy);
         } else if (st == kStCol0 || st == kStCol1) {
             // v: lane = y, register kx.  Transpose to lane = kx, register
             // bitrev(y).  REAL mode: column kx = 0 of Z is zeroed here, so
@@ -333,28 +493,26 @@ __device__ __forceinline__ void fp32_task(const PivParams& p, const int task, fl
                 v[0] = make_float2(0.f, 0.f);
                 v[W / 2] = make_float2(0.f, 0.f);
             }
+            // the product at (ky, kx) is the conjugate of that at (-ky, -kx):
+            // a lane takes rows ky <= W/2 of its column, with the mirrored
+            // bin from lane -kx, and writes the mirrored Q too
             const int pl = (W - gl) & (W - 1);
-            // first window: its product goes to the half spectrum H (lanes
-            // kx <= W/2); second window: lanes kx > W/2 take the first product
-            // from the mirror (-ky, W - kx) of H, conjugated, and Q goes to S
-            const bool mirror = gl > W / 2;
-            const int hc = mirror ? W - gl : gl;
-            const float sg = mirror ? -1.f : 1.f;
-            const bool store_h = (h == 0) && !mirror;
-#pragma unroll
-            for (int ky = 0; ky < W; ++ky) {
-                const int mky = (W - ky) & (W - 1);
+            auto product = [&](int ky) -> float2 {   // 4 conj(P)
                 const float2 z = v[ky];
-                const float zmx = __shfl_sync(0xffffffffu, v[mky].x, pl, W);
-                const float zmy = __shfl_sync(0xffffffffu, v[mky].y, pl, W);
-                // 4 conj(P) = ( 2 Im(Z Zm), |Z|^2 - |Zm|^2 )
-                const float im2 = 2.f * fmaf(z.x, zmy, z.y * zmx);
-                const float d = fmaf(z.x, z.x, fmaf(z.y, z.y, -fmaf(zmx, zmx, zmy * zmy)));
-                if (store_h) H[hix<W>(ky, gl)] = make_float2(im2, d);
-                if (h == 1) {
+                const float2 m = make_float2(__shfl_sync(0xffffffffu, v[(W - ky) & (W - 1)].x, pl, W),
+                                             __shfl_sync(0xffffffffu, v[(W - ky) & (W - 1)].y, pl, W));
+                return four_conj_p(z, m);
+            };
+            if (h == 0) {
+#pragma unroll
+                for (int ky = 0; ky <= W / 2; ++ky) H[ky * W + gl] = product(ky);
+            } else {
+#pragma unroll
+                for (int ky = 0; ky <= W / 2; ++ky) {
                     // Q = conj(4 P1) + i conj(4 P2), stored at [ky][kx]
-                    const float2 c1 = H[hix<W>(mirror ? mky : ky, hc)];
-                    S[tix<W>(ky, gl)] = make_float2(c1.x - d, fmaf(sg, c1.y, im2));
+                    const float2 c1 = H[ky * W + gl], c2 = product(ky);
+                    S[tix<W>(ky, gl)] = make_float2(c1.x - c2.y, c1.y + c2.x);
+                    if (ky > 0 && ky < W / 2) S[tix<W>(W - ky, pl)] = make_float2(c1.x + c2.y, c2.x - c1.y);
                 }
             }
             __syncwarp();
@@ -363,157 +521,173 @@ __device__ __forceinline__ void fp32_task(const PivParams& p, const int task, fl
     // v: lane = x, register y; v.x = plane of the first window of the pair,
     // v.y of the second (4x scaled, pedestal removed).
 
-    const float dlt = p.kappa * 5.9604645e-8f * 2.f * (float)N * (en0 + en1);
+    const float dlt = p.kappa * 5.9604645e-8f * 2.f * (float)N * group_sum<W, float>(energy.x + energy.y);
     const int xs = (gl + W / 2) & (W - 1);          // swapped column of this lane
-    const bool col_ok = xs >= SX0 && xs < SX1;
 
+    // plane rows y into shared memory (row-major, padded), row 0 again after
+    // the last (H is free)
+#pragma unroll
+    for (int y = 0; y < W; ++y) S[tix<W>(y, gl)] = v[y];
+    S[tix<W>(W, gl)] = v[0];
+    if (PLANES) {
 #pragma unroll 1
-    for (int h = 0; h < 2; ++h) {
-        const int w = first + h * NG + grp;
-        const bool valid = w < (int)p.n_win;
-        if (h == 1) {                                // the second plane into .x
-#pragma unroll
-            for (int i = 0; i < W; ++i) v[i].x = v[i].y;
-        }
-
-        // plane rows y into shared memory (row-major, padded) for the fit
-#pragma unroll
-        for (int y = 0; y < W; ++y) S[tix<W>(y, gl)].x = v[y].x;
-        if (PLANES && valid) {
-#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int w = first + h * NG + grp;
+            if (w >= (int)p.n_win) continue;
             for (int y = 0; y < W; ++y) {
-                const int ys = (y + W / 2) & (W - 1);
-                p.planes[(size_t)w * N + ys * W + xs] = 0.25f * v[y].x;
+                const float2 c = S[tix<W>(y, gl)];   // the lane's own column
+                p.planes[(size_t)w * N + ((y + W / 2) & (W - 1)) * W + xs] = 0.25f * (h ? c.y : c.x);
             }
         }
+    }
+    __syncwarp();
 
-        // ---- find_peaks: strict 4-neighbour maxima, top two
-        float t0 = kNegInf, t1 = kNegInf, umax = kNegInf;
-        int t0y = 0;
+    // ---- find_peaks on both planes: strict 4-neighbour maxima, top two.
+    // The columns beside the lane's come from the tile: one 64-bit load is
+    // both planes' neighbour, where a shuffle is one plane's.  16 px: the
+    // lane's own column from its registers, fully unrolled.  32 px: from the
+    // tile too, in a loop of a few rows: unrolled, 29 rows are a third of the
+    // kernel's code, and fetching it held up 1.0 warps an issue (0.2 in the
+    // loop: 751 -> 709 us for a 4096 x 4096 pair at step 8; a 2048 x 1536 pass of
+    // 16 px windows takes 42.0 us in the loop and 40.5 without).
+    Top2 s[2];
+    s[0].init();
+    s[1].init();
+    {
+        const int gl_l = (gl + W - 1) & (W - 1), gl_r = (gl + 1) & (W - 1);
+        auto row = [&](float2 up, float2 c, float2 dn, const float2* at, int ys) {   // at: the row in the tile
+            const float2 l = at[gl_l], r = at[gl_r];
+            s[0].add(c.x, max4(up.x, dn.x, l.x, r.x), dlt, ys);
+            s[1].add(c.y, max4(up.y, dn.y, l.y, r.y), dlt, ys);
+        };
+        if constexpr (W == 16) {
 #pragma unroll
-        for (int ys = SY0; ys < SY1; ++ys) {
-            const int y = (ys + W / 2) & (W - 1);
-            const float c = v[y].x;
-            const float up = v[(y + W - 1) & (W - 1)].x;
-            const float dn = v[(y + 1) & (W - 1)].x;
-            const float lf = __shfl_sync(0xffffffffu, c, (gl + W - 1) & (W - 1), W);
-            const float rt = __shfl_sync(0xffffffffu, c, (gl + 1) & (W - 1), W);
-            float m4;   // max of the four neighbours (a three-source max and a max)
-            asm("max.f32 %0, %1, %2, %3;" : "=f"(m4) : "f"(up), "f"(dn), "f"(fmaxf(lf, rt)));
-            const float dd = m4 - c;
-            const bool strict = col_ok && (dd < 0.f);
-            const bool unc = col_ok && (fabsf(dd) <= dlt);
-            umax = unc ? fmaxf(umax, c) : umax;
-            const float sv = strict ? c : kNegInf;
-            const bool gt = sv > t0;
-            t1 = gt ? t0 : fmaxf(t1, sv);
-            t0y = gt ? ys : t0y;
-            t0 = gt ? sv : t0;
+            for (int ys = SY0; ys < SY1; ++ys) {
+                const int y = (ys + W / 2) & (W - 1);
+                row(v[(y + W - 1) & (W - 1)], v[y], v[(y + 1) & (W - 1)], S + tix<W>(y, 0), ys);
+            }
+        } else {
+            float2 up = S[tix<W>(SY0 + W / 2 - 1, gl)], c = S[tix<W>(SY0 + W / 2, gl)];
+            auto rows = [&](const float2* at, int ys0, int ys1) {
+#pragma unroll 2
+                for (int ys = ys0; ys < ys1; ++ys, at += W + 1) {
+                    const float2 dn = at[W + 1 + gl];
+                    row(up, c, dn, at, ys);
+                    up = c;
+                    c = dn;
+                }
+            };
+            rows(S + tix<W>(SY0 + W / 2, 0), SY0, W / 2);
+            rows(S, W / 2, SY1);
         }
-        int key = t0y * W + xs;                     // row-major index in the swapped plane
+        s[0].key = s[0].key * W + xs;   // row-major index in the swapped plane
+        s[1].key = s[1].key * W + xs;
+        if (xs < SX0 || xs >= SX1) {
+            s[0].init();
+            s[1].init();
+        }
+    }
+
+    // ---- half of the group's lanes to each plane: reduction, fit, result
+    constexpr int HL = W / 2;
+    const int h = gl / HL, hl = gl % HL;
+    const int w = first + h * NG + grp;
+    Top2 g = h ? s[1] : s[0];
+    {
+        const Top2 other = h ? s[0] : s[1];
+        g.merge(other.across(HL));
+    }
 #pragma unroll
-        for (int o = W / 2; o > 0; o >>= 1) {
-            const float o0 = __shfl_xor_sync(0xffffffffu, t0, o, W);
-            const float o1 = __shfl_xor_sync(0xffffffffu, t1, o, W);
-            const int ok = __shfl_xor_sync(0xffffffffu, key, o, W);
-            const bool take = (o0 > t0) || (o0 == t0 && ok < key);
-            const float n1 = take ? fmaxf(t0, o1) : fmaxf(t1, o0);
-            t0 = take ? o0 : t0;
-            key = take ? ok : key;
-            t1 = n1;
-        }
-        umax = group_max<W>(umax);
-        __syncwarp();
+    for (int o = HL / 2; o > 0; o >>= 1) g.merge(g.across(o));
 
-        // ---- fit_simple_gaussian: the six logarithms on six lanes
-        const int px = key % W, py = key / W;       // swapped-plane coordinates
-        const int ux = (px + W / 2) & (W - 1), uy = (py + W / 2) & (W - 1);
-        const float ped = h ? ped1 : ped0;
-        const float vc = S[tix<W>(uy, ux)].x;
-        const float vl = S[tix<W>(uy, (ux + W - 1) & (W - 1))].x;
-        const float vr = S[tix<W>(uy, (ux + 1) & (W - 1))].x;
-        const float vu = S[tix<W>((uy + W - 1) & (W - 1), ux)].x;
-        const float vd = S[tix<W>((uy + 1) & (W - 1), ux)].x;
-        __syncwarp();
-        // axis x: ln(L/R), ln(L/C), ln(R/C); axis y: ln(U/D), ln(U/C), ln(D/C)
-        // with L = vl + ped etc., each as log1p((num - den) / (den + ped))
-        const int j = gl < 6 ? gl : 0;
-        const float an = j == 0 ? vl : j == 1 ? vl : j == 2 ? vr : j == 3 ? vu : j == 4 ? vu : vd;
-        const float ad = j == 0 ? vr : j == 1 ? vc : j == 2 ? vc : j == 3 ? vd : vc;
-        const float lg = log1pf((an - ad) / (ad + ped));
-        const float lxr = __shfl_sync(0xffffffffu, lg, 0, W);
-        const float lxl = __shfl_sync(0xffffffffu, lg, 1, W);
-        const float lxrr = __shfl_sync(0xffffffffu, lg, 2, W);
-        const float lyd = __shfl_sync(0xffffffffu, lg, 3, W);
-        const float lyu = __shfl_sync(0xffffffffu, lg, 4, W);
-        const float lydd = __shfl_sync(0xffffffffu, lg, 5, W);
+    const bool has2 = g.t1 > kNegInf;
+    const int px = has2 ? g.key % W : HL, py = has2 ? g.key / W : HL;       // swapped-plane coordinates
+    const int ux = (px + W / 2) & (W - 1), uy = (py + W / 2) & (W - 1);
+    const float ped = h ? ped1 : ped0;
+    auto cell = [&](int y, int x) -> float {
+        const float2 c = S[tix<W>(y & (W - 1), x & (W - 1))];
+        return h ? c.y : c.x;
+    };
+    const float vc = cell(uy, ux), vl = cell(uy, ux + W - 1), vr = cell(uy, ux + 1);
+    const float vu = cell(uy + W - 1, ux), vd = cell(uy + 1, ux);
+    // fit_simple_gaussian, the six logarithms on six lanes.
+    // axis x: ln(L/R), ln(L/C), ln(R/C); axis y: ln(U/D), ln(U/C), ln(D/C)
+    // with L = vl + ped etc., each as log1p((num - den) / (den + ped))
+    const int j = hl < 6 ? hl : 0;
+    const float an = j == 0 ? vl : j == 1 ? vl : j == 2 ? vr : j == 3 ? vu : j == 4 ? vu : vd;
+    const float ad = j == 0 ? vr : j == 1 ? vc : j == 2 ? vc : j == 3 ? vd : vc;
+    const float lg = log1pf((an - ad) / (ad + ped));
+    const float lxr = __shfl_sync(0xffffffffu, lg, 0, HL);
+    const float lxl = __shfl_sync(0xffffffffu, lg, 1, HL);
+    const float lxrr = __shfl_sync(0xffffffffu, lg, 2, HL);
+    const float lyd = __shfl_sync(0xffffffffu, lg, 3, HL);
+    const float lyu = __shfl_sync(0xffffffffu, lg, 4, HL);
+    const float lydd = __shfl_sync(0xffffffffu, lg, 5, HL);
 
-        int slot = -1;
-        if (valid && gl == 0) {
-            const bool has2 = t1 > kNegInf;
-            bool certain;
-            opiv_vector out{ 0.f, 0.f, 0.f, 0.f, 0.f };
-            int32_t code = -1;
-            int bx, by, ox, oy;
-            window_origin(p, w, bx, by);
-            b_offset(p, W, bx, by, ox, oy);
-            if (!has2) {
-                certain = !(umax > kNegInf);
-            } else {
-                const float C = vc + ped, L = vl + ped, R = vr + ped, U = vu + ped, D = vd + ped;
-                const float nan = __int_as_float(0x7fffffff);
-                // (ln L - ln R) / (2 (ln L + ln R - 2 ln C)), NaN where the
-                // reference takes the log of a non-positive value
-                const float denx = lxl + lxrr, deny = lyu + lydd;
-                const bool okx = L > 0.f && C > 0.f && R > 0.f;
-                const bool oky = U > 0.f && C > 0.f && D > 0.f;
-                const float fx = okx ? lxr / (2.f * denx) : nan;
-                const float fy = oky ? lyd / (2.f * deny) : nan;
-                // error bound of each axis for an error dlt/2 per value; a
-                // NaN outcome is certain only if a value is clearly negative
-                const float mx = fminf(fminf(L, R), C), my = fminf(fminf(U, D), C);
-                const float ex = okx ? (denx == 0.f ? 3.4e38f
-                                        : dlt * (1.f + 4.f * fabsf(fx)) / (mx * 2.f * fabsf(denx)))
-                                     : (mx < -dlt ? 0.f : 3.4e38f);
-                const float ey = oky ? (deny == 0.f ? 3.4e38f
-                                        : dlt * (1.f + 4.f * fabsf(fy)) / (my * 2.f * fabsf(deny)))
-                                     : (my < -dlt ? 0.f : 3.4e38f);
-                const float p0 = t0 + ped, p1 = t1 + ped;
-                // sn = p0 / p1 when p1 > 0: relative error <= e/|p0| + e/|p1|
-                // with e = dlt / 2 the error of one plane value
-                const float sn_err = 0.5f * dlt * (1.f / fabsf(p0) + 1.f / fabsf(p1));
-                certain = (umax < t1 - 2.f * dlt) && (t0 - t1 > dlt) && (fabsf(p1) > dlt) &&
-                          (ex < kFitTol) && (ey < kFitTol) &&
-                          (p1 <= 0.f || sn_err < kSnTol * (1.f + p0 / p1));
-                out.x = (float)(bx + W / 2);
-                out.y = (float)(p.img_h - (by + W / 2));
-                out.u = (float)(W / 2 - px - ox) - fx;
-                out.v = (float)(W / 2 - py - oy) - fy;
-                out.sn = (p1 > 0.f) ? p0 / p1 : 0.f;
-                code = key;
-            }
-            p.out_vec[w] = out;
-            if (p.out_peak) p.out_peak[w] = code;
-            if (p.out_disp)
-                p.out_disp[w] = has2 ? pack_disp(px - W / 2 + ox, py - W / 2 + oy) : pack_disp(ox, oy);
-            if (!certain && p.flag_list) {
-                const unsigned int at = atomicAdd(p.flag_count, 1u);
-                p.flag_list[at] = (int32_t)w + p.flag_base;
-                if (at < (unsigned int)p.flag_cap) slot = (int)at;
-            }
+    int slot = -1;
+    if (w < (int)p.n_win && hl == 0) {
+        bool certain;
+        opiv_vector out{ 0.f, 0.f, 0.f, 0.f, 0.f };
+        int32_t code = -1;
+        int bx, by, ox, oy;
+        window_origin(p, w, bx, by);
+        b_offset(p, W, bx, by, ox, oy);
+        if (!has2) {
+            certain = !(g.umax > kNegInf);
+        } else {
+            const float C = vc + ped, L = vl + ped, R = vr + ped, U = vu + ped, D = vd + ped;
+            const float nan = __int_as_float(0x7fffffff);
+            // (ln L - ln R) / (2 (ln L + ln R - 2 ln C)), NaN where the
+            // reference takes the log of a non-positive value
+            const float denx = lxl + lxrr, deny = lyu + lydd;
+            const bool okx = L > 0.f && C > 0.f && R > 0.f;
+            const bool oky = U > 0.f && C > 0.f && D > 0.f;
+            const float fx = okx ? lxr / (2.f * denx) : nan;
+            const float fy = oky ? lyd / (2.f * deny) : nan;
+            // error bound of each axis for an error dlt/2 per value; a
+            // NaN outcome is certain only if a value is clearly negative
+            const float mx = fminf(fminf(L, R), C), my = fminf(fminf(U, D), C);
+            const float ex = okx ? (denx == 0.f ? 3.4e38f
+                                    : dlt * (1.f + 4.f * fabsf(fx)) / (mx * 2.f * fabsf(denx)))
+                                 : (mx < -dlt ? 0.f : 3.4e38f);
+            const float ey = oky ? (deny == 0.f ? 3.4e38f
+                                    : dlt * (1.f + 4.f * fabsf(fy)) / (my * 2.f * fabsf(deny)))
+                                 : (my < -dlt ? 0.f : 3.4e38f);
+            const float p0 = g.t0 + ped, p1 = g.t1 + ped;
+            // sn = p0 / p1 when p1 > 0: relative error <= e/|p0| + e/|p1|
+            // with e = dlt / 2 the error of one plane value
+            const float sn_err = 0.5f * dlt * (1.f / fabsf(p0) + 1.f / fabsf(p1));
+            certain = (g.umax < g.t1 - 2.f * dlt) && (g.t0 - g.t1 > dlt) && (fabsf(p1) > dlt) &&
+                      (ex < kFitTol) && (ey < kFitTol) &&
+                      (p1 <= 0.f || sn_err < kSnTol * fminf(1.f + p0 / p1, kSnCap));
+            out.x = (float)(bx + W / 2);
+            out.y = (float)(p.img_h - (by + W / 2));
+            out.u = (float)(W / 2 - px - ox) - fx;
+            out.v = (float)(W / 2 - py - oy) - fy;
+            out.sn = (p1 > 0.f) ? p0 / p1 : 0.f;
+            code = g.key;
         }
-        // a flagged window hands its plane on (each lane its own column)
-        if (!PLANES) slot = __shfl_sync(0xffffffffu, slot, 0, W);
-        if (!PLANES && slot >= 0) {
-            float* rec = p.flag_planes + (size_t)slot * flag_record_floats(W);
-#pragma unroll 4
-            for (int y = 0; y < W; ++y) rec[((y + W / 2) & (W - 1)) * W + xs] = S[tix<W>(y, gl)].x;
-            if (gl == 0) rec[N] = dlt;
+        p.out_vec[w] = out;
+        if (p.out_peak) p.out_peak[w] = code;
+        if (p.out_disp)
+            p.out_disp[w] = has2 ? pack_disp(px - W / 2 + ox, py - W / 2 + oy) : pack_disp(ox, oy);
+        if (!certain && p.flag_list) {
+            const unsigned int at = atomicAdd(p.flag_count, 1u);
+            p.flag_list[at] = (int32_t)w + p.flag_base;
+            if (at < (unsigned int)p.flag_cap) slot = (int)at;
         }
+    }
+    // a flagged window hands its plane on
+    if (!PLANES) slot = __shfl_sync(0xffffffffu, slot, 0, HL);
+    if (!PLANES && slot >= 0) {
+        float* rec = p.flag_planes + (size_t)slot * flag_record_floats(W);
+#pragma unroll 1
+        for (int i = hl; i < N; i += HL) rec[i] = cell(i / W + W / 2, i % W + W / 2);
+        if (hl == 0) rec[N] = dlt;
     }
 }
 
-extern __shared__ float2 fp32_dyn_smem[];
+extern __shared__ __align__(16) float2 fp32_dyn_smem[];   // rows are staged in 16-byte blocks
 
 // resident CTAs per SM the register budget is set for: a 16 px window's
 // transform needs half the registers of a 32 px one

@@ -60,6 +60,7 @@ constexpr int kCtasPerSm = 4;
 // certification thresholds: as the 16 / 32 px kernel (piv_fp32.cuh)
 constexpr float kFitTol = 6e-5f;
 constexpr float kSnTol = 6e-6f;
+constexpr float kSnCap = 4.f;
 #define kNegInf64 (-__int_as_float(0x7f800000))
 
 // base-8 digit reversal of a 6-bit index (an involution)
@@ -68,32 +69,6 @@ __device__ __forceinline__ int dr(int v) { return ((v & 7) << 3) | (v >> 3); }
 __device__ __forceinline__ float2 cmul(float2 a, float2 w)
 {
     return make_float2(fmaf(a.x, w.x, -a.y * w.y), fmaf(a.x, w.y, a.y * w.x));
-}
-
-// Packed FP32 pairs (one instruction for both components; each rounds as the
-// scalar one does).
-__device__ __forceinline__ float2 add2(float2 a, float2 b)
-{
-    float2 d;
-    asm("{ .reg .b64 x, y; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; add.rn.f32x2 x, x, y; mov.b64 {%0, %1}, x; }"
-        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return d;
-}
-__device__ __forceinline__ float2 sub2(float2 a, float2 b)
-{
-    float2 d;
-    asm("{ .reg .b64 x, y; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; sub.rn.f32x2 x, x, y; mov.b64 {%0, %1}, x; }"
-        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return d;
-}
-
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
-{
-    float2 d;
-    asm("{ .reg .b64 x, y, z; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; mov.b64 z, {%6, %7}; "
-        "fma.rn.f32x2 x, x, y, z; mov.b64 {%0, %1}, x; }"
-        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-    return d;
 }
 
 // In-place forward 8-point DFT, natural order in and out.
@@ -187,10 +162,8 @@ struct pair_slot {
 };
 __device__ __forceinline__ pair_slot product(float2 z, float2 m)
 {
-    pair_slot s;
-    s.im = 2.f * fmaf(z.x, m.y, z.y * m.x);
-    s.d = fmaf(z.x, z.x, fmaf(z.y, z.y, -fmaf(m.x, m.x, m.y * m.y)));
-    return s;
+    const float2 p = four_conj_p(z, m);
+    return pair_slot{ p.x, p.y };
 }
 // Q = conj(4 P1) + i conj(4 P2) at A's bin and at its mirror
 __device__ __forceinline__ float2 q_at(pair_slot a, pair_slot b) { return make_float2(a.im - b.d, a.d + b.im); }
@@ -591,7 +564,7 @@ __device__ __forceinline__ void w64_task(const PivParams& p, const int blk)
                 const float sn_err = 0.5f * dlt * (1.f / fabsf(p0) + 1.f / fabsf(p1));
                 certain = (g.umax < g.t1 - 2.f * dlt) && (g.t0 - g.t1 > dlt) && (fabsf(p1) > dlt) &&
                           (ex < kFitTol) && (ey < kFitTol) &&
-                          (p1 <= 0.f || sn_err < kSnTol * (1.f + p0 / p1));
+                          (p1 <= 0.f || sn_err < kSnTol * fminf(1.f + p0 / p1, kSnCap));
                 out.x = (float)(bx + W / 2);
                 out.y = (float)(p.img_h - (by + W / 2));
                 out.u = (float)(W / 2 - px - ox) - fx;
