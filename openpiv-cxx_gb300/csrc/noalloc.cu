@@ -59,7 +59,7 @@ namespace {
 
 constexpr int64_t kNoAllocMaxWindows = 1 << 20;
 // byte layout of the scratch array
-constexpr size_t kOffCount = 0;                                   // unsigned int
+constexpr size_t kOffCount = 0;                                   // kFlagCounters unsigned ints
 constexpr size_t kOffList = 256;                                  // int32 x max windows
 constexpr size_t kOffTw16 = kOffList + 4 * (size_t)kNoAllocMaxWindows;   // double2 x 2*16
 constexpr size_t kOffTw32 = kOffTw16 + sizeof(double2) * 2 * 16;          // double2 x 2*32
@@ -193,6 +193,7 @@ extern "C" int opiv_process_pair_device_noalloc(const void* d_frame_a, const voi
     k.kappa = kNoAllocKappa;
     k.flag_count = reinterpret_cast<unsigned int*>(scratch + kOffCount);
     k.flag_list = reinterpret_cast<int32_t*>(scratch + kOffList);
+    k.flag_room = (int32_t)n;
     // planes of flagged windows: what this grid leaves of the list's room
     const size_t used = ((size_t)n * sizeof(int32_t) + 15) / 16 * 16;
     const size_t left = sizeof(int32_t) * (size_t)kNoAllocMaxWindows - std::min(used, sizeof(int32_t) * (size_t)kNoAllocMaxWindows);
@@ -202,7 +203,7 @@ extern "C" int opiv_process_pair_device_noalloc(const void* d_frame_a, const voi
     k.tw_fwd = tw;
     k.tw_rev = tw + ia;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if ((e = cudaMemsetAsync(scratch + kOffCount, 0, sizeof(unsigned int), s)) != cudaSuccess)
+    if ((e = cudaMemsetAsync(scratch + kOffCount, 0, kFlagCounters * sizeof(unsigned int), s)) != cudaSuccess)
         return na_fail(OPIV_ERR_CUDA, "clearing the scratch counter: %s", cudaGetErrorString(e));
     if ((e = launch_piv_fp32(k, (int)ia, dtype, mode, limit_search ? 1 : 0, false, s)) != cudaSuccess)
         return na_fail(OPIV_ERR_CUDA, "FP32 pass: %s", cudaGetErrorString(e));

@@ -192,7 +192,7 @@ struct opiv_plan {
     float* d_flag_planes = nullptr;     // planes of the first flag_cap flagged windows
     int32_t flag_cap = 0;
     double2* d_tw = nullptr;            // forward then reverse, ia entries each
-    unsigned int* h_flag_count = nullptr;   // pinned copy of the last count
+    bool flags = false;                 // the last pass was an FP32 one: d_flag_count[2] is its count
     bool timing = false;
     cudaEvent_t ev[3] = { nullptr, nullptr, nullptr };   // fp32 start, fp32 end, exact end
     int32_t* d_disp = nullptr;          // integer displacements (multi-pass plans)
@@ -264,7 +264,6 @@ void plan_free(opiv_plan* p)
     if (p->up) cudaStreamDestroy(p->up);
     if (p->down) cudaStreamDestroy(p->down);
     if (p->cs2) cudaStreamDestroy(p->cs2);
-    if (p->h_flag_count) cudaFreeHost(p->h_flag_count);
     for (cudaEvent_t& e : p->ev)
         if (e) cudaEventDestroy(e);
     if (p->stream) cudaStreamDestroy(p->stream);
@@ -288,6 +287,7 @@ PivParams base_params(const opiv_plan* p)
     k.flag_list = p->d_flag_list;
     k.flag_planes = p->d_flag_planes;
     k.flag_cap = p->flag_cap;
+    k.flag_room = (int32_t)p->n_win;
     k.tw_fwd = p->d_tw;
     k.tw_rev = p->d_tw + p->ia;
     return k;
@@ -334,7 +334,7 @@ int run_pass(opiv_plan* p, const void* fa, const void* fb, size_t pitch, opiv_ve
         k.flag_list = flag_list;
         k.flag_planes = flag_planes;
     }
-    CUDA_TRY(cudaMemsetAsync(k.flag_count, 0, sizeof(unsigned int), s));
+    if (!flag_count) p->flags = p->precision == OPIV_PREC_FP32;
     if (is_tc(p->precision)) {
         if (((uintptr_t)fa | (uintptr_t)fb | (uintptr_t)pitch) % 16 != 0)
             return fail(OPIV_ERR_ARG, "the tensor-core path needs 16-byte aligned frame rows");
@@ -369,7 +369,12 @@ int run_pass(opiv_plan* p, const void* fa, const void* fb, size_t pitch, opiv_ve
     CUDA_TRY(launch_piv_fp32(k, (int)p->ia, p->dtype, p->mode, p->limit, false, s));
     ++g_launches;
     if (p->timing) CUDA_TRY(cudaEventRecord(p->ev[1], s));
-    CUDA_TRY(launch_piv_exact(k, (int)p->ia, p->dtype, p->mode, p->limit, true, exact_blocks(p->device), s));
+    const cudaError_t e =
+        launch_piv_exact(k, (int)p->ia, p->dtype, p->mode, p->limit, true, exact_blocks(p->device), s);
+    if (e != cudaSuccess) {   // the counters as the next pass wants them
+        cudaMemsetAsync(k.flag_count, 0, kFlagCounters * sizeof(unsigned int), s);
+        return cuda_fail(e, "launch_piv_exact");
+    }
     ++g_launches;
     if (p->timing) CUDA_TRY(cudaEventRecord(p->ev[2], s));
     return OPIV_OK;
@@ -509,7 +514,7 @@ int plan_create(opiv_plan** out, uint32_t img_w, uint32_t img_h, int dtype, uint
         return at;
     };
     const size_t at_vec = part(sizeof(opiv_vector) * p->n_win), at_peak = part(sizeof(int32_t) * p->n_win);
-    const size_t at_count = part(sizeof(unsigned int)), at_list = part(sizeof(int32_t) * p->n_win);
+    const size_t at_count = part(kFlagCounters * sizeof(unsigned int)), at_list = part(sizeof(int32_t) * p->n_win);
     const size_t at_planes = part(flag_plane_bytes(p->flag_cap, ia)), at_tw = part(sizeof(double2) * 2 * ia);
     if ((e = cudaMalloc(&p->d_scratch, bytes)) != cudaSuccess) return done(cuda_fail(e, "cudaMalloc(plan scratch)"));
     p->d_vec = reinterpret_cast<opiv_vector*>(p->d_scratch + at_vec);
@@ -518,11 +523,8 @@ int plan_create(opiv_plan** out, uint32_t img_w, uint32_t img_h, int dtype, uint
     p->d_flag_list = reinterpret_cast<int32_t*>(p->d_scratch + at_list);
     p->d_flag_planes = reinterpret_cast<float*>(p->d_scratch + at_planes);
     p->d_tw = reinterpret_cast<double2*>(p->d_scratch + at_tw);
-    if ((e = cudaMemset(p->d_flag_count, 0, sizeof(unsigned int))) != cudaSuccess)
+    if ((e = cudaMemsetAsync(p->d_flag_count, 0, kFlagCounters * sizeof(unsigned int), p->stream)) != cudaSuccess)
         return done(cuda_fail(e, "cudaMemset"));
-    if ((e = cudaMallocHost(&p->h_flag_count, sizeof(unsigned int))) != cudaSuccess)
-        return done(cuda_fail(e, "cudaMallocHost"));
-    *p->h_flag_count = 0;
     if (is_pow2(ia)) {   // the exact kernel's twiddles (FFT path)
         std::vector<double2> tw = reference_twiddles(ia, -1), tr = reference_twiddles(ia, +1);
         tw.insert(tw.end(), tr.begin(), tr.end());
@@ -530,6 +532,8 @@ int plan_create(opiv_plan** out, uint32_t img_w, uint32_t img_h, int dtype, uint
             cudaSuccess)
             return done(cuda_fail(e, "cudaMemcpy(twiddles)"));
     }
+    // passes on any stream rely on the counters
+    if ((e = cudaStreamSynchronize(p->stream)) != cudaSuccess) return done(cuda_fail(e, "cudaStreamSynchronize"));
     return done(OPIV_OK);
 }
 
@@ -593,9 +597,6 @@ int opiv_process_pair_device(opiv_plan* plan, const void* d_fa, const void* d_fb
     cudaSetDevice(plan->device);
     const int rc = run_pass(plan, d_fa, d_fb, pitch_bytes, d_out_vec, d_out_peak,
                             (cudaStream_t)stream);
-    if (rc == OPIV_OK)
-        cudaMemcpyAsync(plan->h_flag_count, plan->d_flag_count, sizeof(unsigned int),
-                        cudaMemcpyDeviceToHost, (cudaStream_t)stream);
     cudaSetDevice(prev);
     return rc;
 }
@@ -635,8 +636,6 @@ int opiv_process_pair(opiv_plan* plan, const void* frame_a, const void* frame_b,
         (e = cudaMemcpyAsync(out_peak, plan->d_peak, sizeof(int32_t) * plan->n_win,
                              cudaMemcpyDeviceToHost, s)) != cudaSuccess)
         return done(cuda_fail(e, "cudaMemcpyAsync(peaks)"));
-    cudaMemcpyAsync(plan->h_flag_count, plan->d_flag_count, sizeof(unsigned int),
-                    cudaMemcpyDeviceToHost, s);
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess)
         return done(cuda_fail(e, "cudaStreamSynchronize"));
     if (plan->d_status) return done(opiv_plan_status(plan));
@@ -669,11 +668,15 @@ int opiv_process_pairs(opiv_plan* plan, int64_t n_pairs, const void* const* fram
             if ((e = cudaEventCreateWithFlags(&plan->ev_up[k], cudaEventDisableTiming)) != cudaSuccess) break;
             if ((e = cudaEventCreateWithFlags(&plan->ev_done[k], cudaEventDisableTiming)) != cudaSuccess) break;
             if ((e = cudaEventCreateWithFlags(&plan->ev_down[k], cudaEventDisableTiming)) != cudaSuccess) break;
-            if ((e = cudaMalloc(&plan->p_flag_count[k], sizeof(unsigned int))) != cudaSuccess) break;
+            if ((e = cudaMalloc(&plan->p_flag_count[k], kFlagCounters * sizeof(unsigned int))) != cudaSuccess) break;
+            if ((e = cudaMemsetAsync(plan->p_flag_count[k], 0, kFlagCounters * sizeof(unsigned int), plan->stream)) !=
+                cudaSuccess)
+                break;
             if ((e = cudaMalloc(&plan->p_flag_list[k], sizeof(int32_t) * plan->n_win)) != cudaSuccess) break;
             if (plan->flag_cap > 0)
                 e = cudaMalloc(&plan->p_flag_planes[k], flag_plane_bytes(plan->flag_cap, plan->ia));
         }
+        if (e == cudaSuccess) e = cudaStreamSynchronize(plan->stream);   // both compute streams rely on the counters
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&plan->up, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&plan->down, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&plan->cs2, cudaStreamNonBlocking);
@@ -732,8 +735,16 @@ int opiv_process_pairs(opiv_plan* plan, int64_t n_pairs, const void* const* fram
 int64_t opiv_plan_exact_count(opiv_plan* plan)
 {
     if (!plan) return fail(OPIV_ERR_ARG, "plan is null");
+    unsigned int count = 0;
+    if (!plan->flags) return 0;   // the other precisions flag nothing
+    int prev = 0;
+    cudaGetDevice(&prev);
+    cudaSetDevice(plan->device);
     cudaDeviceSynchronize();
-    return (int64_t)*plan->h_flag_count;
+    const cudaError_t e = cudaMemcpy(&count, plan->d_flag_count + 2, sizeof count, cudaMemcpyDeviceToHost);
+    cudaSetDevice(prev);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpy(flag count)");
+    return (int64_t)count;
 }
 
 int opiv_multipass_create(opiv_multipass** out, uint32_t img_w, uint32_t img_h, int dtype,
@@ -1046,6 +1057,7 @@ int batch_queue_setup(opiv_batch* b)
                 pq.items[j].flag_list = q.d_flags + flag_off[g];
                 pq.items[j].flag_planes = q.d_planes + plane_off[g] * flag_record_floats(q.ia);
                 pq.items[j].flag_cap = (int32_t)(plane_off[g + 1] - plane_off[g]);
+                pq.items[j].flag_room = (int32_t)(flag_off[g + 1] - flag_off[g]);
             }
             pq.items_g = q.d_items + (size_t)kQueueMaxItems * g;
             pq.task_item = q.d_task_item + task_off[g];

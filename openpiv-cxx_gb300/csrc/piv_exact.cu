@@ -557,7 +557,7 @@ piv_exact_kernel(const PivParams p, int W, int mode, int limit)
     extern __shared__ double2 sm[];
     __shared__ int row_count[kMaxW];
     __shared__ int total_cand;
-    const int64_t nwork = LIST ? (int64_t)(*p.flag_count) : p.n_win;
+    const int64_t nwork = LIST ? (int64_t)min(*p.flag_count, (unsigned int)p.flag_room) : p.n_win;
     int sy0, sy1, sx0, sx1;
     scan_range(W, limit, sy0, sy1, sx0, sx1);
     for (int64_t item = blockIdx.x; item < nwork; item += gridDim.x) {
@@ -571,6 +571,17 @@ piv_exact_kernel(const PivParams p, int W, int mode, int limit)
                 continue;
         }
         exact_window<PixT>(p, w, W, mode, sy0, sy1, sx0, sx1, sm, sm + W * W, row_count, &total_cand);
+    }
+    if constexpr (LIST) {
+        // the last CTA to finish leaves the counters as the next pass wants
+        // them (every CTA has read the count by then), so that a pass is two
+        // launches: a memset before them and a copy of the count after them
+        // were half of a small pass's time (160 x 128 px: 25.8 -> XXX us)
+        if (threadIdx.x == 0 && atomicAdd(p.flag_count + 1, 1u) == gridDim.x - 1) {
+            p.flag_count[2] = (unsigned int)nwork;
+            p.flag_count[1] = 0u;
+            p.flag_count[0] = 0u;
+        }
     }
 }
 

@@ -578,7 +578,7 @@ __device__ __forceinline__ void w64_task(const PivParams& p, const int blk)
                 p.out_disp[w] = has2 ? pack_disp(px - W / 2 + ox, py - W / 2 + oy) : pack_disp(ox, oy);
             if (!certain && p.flag_list) {
                 const unsigned int at = atomicAdd(p.flag_count, 1u);
-                p.flag_list[at] = (int32_t)w + p.flag_base;
+                if (at < (unsigned int)p.flag_room) p.flag_list[at] = (int32_t)w + p.flag_base;
                 if (at < (unsigned int)p.flag_cap) slot = (int)at;
             }
         }

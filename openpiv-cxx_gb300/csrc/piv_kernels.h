@@ -11,7 +11,7 @@ enum { kModeReal = OPIV_CORR_REAL, kModeComplex = OPIV_CORR_COMPLEX };
 enum { kU8 = OPIV_U8, kU16 = OPIV_U16, kF32 = OPIV_F32, kF64 = 3 /* internal: batch API */ };
 
 // Everything one pass over an image pair needs on the device.
-struct PivParams {
+struct alignas(16) PivParams {
     const void* fa = nullptr;          // frame A (device), img_h rows of `pitch` bytes
     const void* fb = nullptr;          // frame B
     size_t pitch = 0;                  // bytes per row
@@ -26,7 +26,10 @@ struct PivParams {
     int64_t n_win = 0;
     opiv_vector* out_vec = nullptr;
     int32_t* out_peak = nullptr;       // may be null
-    // windows whose FP32 decisions are not certain (see piv_fp32.cu)
+    // windows whose FP32 decisions are not certain (see piv_fp32.cu).  The
+    // single-pair passes' flag_count is kFlagCounters counters, zero before a
+    // pass: windows flagged, and the exact launch's, which leaves them zero
+    // (a queue's is one counter, reset by its launcher).
     unsigned int* flag_count = nullptr;
     int32_t* flag_list = nullptr;
     int32_t flag_base = 0;             // added to a flagged window's index (a queue's list)
@@ -34,6 +37,7 @@ struct PivParams {
     // list: flag_record_floats(W) floats each, the quadrant-swapped FP32
     // plane and then its error bound (refine_window in piv_exact.cu)
     int32_t flag_cap = 0;
+    int32_t flag_room = 0;             // entries of flag_list
     float* flag_planes = nullptr;
     float kappa = 16.f;                // FP32 error-bound factor
     // debug / per-window API outputs
@@ -55,6 +59,10 @@ struct PivParams {
     int32_t* out_disp = nullptr;       // this pass's integer displacements (may be null)
     int* status = nullptr;             // tensor-core kernel: set to 1 if an MMA wait gave up
 };
+
+// flag_count[0]: windows flagged so far; [1]: CTAs of the exact launch that
+// are done; [2]: windows flagged in the last pass.
+constexpr int kFlagCounters = 3;
 
 // Floats of a flagged window's record: the plane, its error bound, padding
 // to 16 bytes.
@@ -161,7 +169,7 @@ struct PivQueue {
     const int32_t* flag_list = nullptr;
 };
 static_assert(kQueueMaxItems <= 256, "task_item holds pair numbers in one byte");
-static_assert(sizeof(PivParams) == 224, "descriptor size (queue parameter space)");
+static_assert(sizeof(PivParams) == 240, "descriptor size (queue parameter space)");
 static_assert(sizeof(PivParams) % 16 == 0, "descriptors are copied in 16-byte words");
 // tasks of a pair of n_win windows in the queue of window size w
 inline int fp32_queue_tasks(int w, int64_t n_win)
