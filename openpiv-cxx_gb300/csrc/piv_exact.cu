@@ -576,7 +576,7 @@ piv_exact_kernel(const PivParams p, int W, int mode, int limit)
         // the last CTA to finish leaves the counters as the next pass wants
         // them (every CTA has read the count by then), so that a pass is two
         // launches: a memset before them and a copy of the count after them
-        // were half of a small pass's time (160 x 128 px: 25.8 -> XXX us)
+        // were half of a small pass's time (160 x 128 px: 25.8 -> 14.3 us)
         if (threadIdx.x == 0 && atomicAdd(p.flag_count + 1, 1u) == gridDim.x - 1) {
             p.flag_count[2] = (unsigned int)nwork;
             p.flag_count[1] = 0u;
