@@ -557,6 +557,7 @@ piv_exact_kernel(const PivParams p, int W, int mode, int limit)
     extern __shared__ double2 sm[];
     __shared__ int row_count[kMaxW];
     __shared__ int total_cand;
+    if (LIST) after_previous();
     const int64_t nwork = LIST ? (int64_t)min(*p.flag_count, (unsigned int)p.flag_room) : p.n_win;
     int sy0, sy1, sx0, sx1;
     scan_range(W, limit, sy0, sy1, sx0, sx1);
@@ -633,6 +634,8 @@ cudaError_t launch_t(const PivParams& p, int w, int mode, int limit, int blocks,
         if (e != cudaSuccess) return e;
         attr_done.fetch_or(bit);
     }
+    if (LIST)
+        return launch_dependent(piv_exact_kernel<PixT, LIST>, (unsigned)blocks, kThreads, smem, s, p, w, mode, limit);
     piv_exact_kernel<PixT, LIST><<<blocks, kThreads, smem, s>>>(p, w, mode, limit);
     return cudaGetLastError();
 }

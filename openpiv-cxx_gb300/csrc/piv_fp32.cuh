@@ -698,6 +698,7 @@ template <int W, int MODE, bool LIMIT, typename PixT, bool PLANES, bool VEC>
 __global__ void __launch_bounds__(32 * kWarps, min_ctas<W>())
 piv_fp32_kernel(const PivParams p)
 {
+    after_previous();
     fp32_task<W, MODE, LIMIT, PixT, PLANES, VEC>(p, (int)blockIdx.x * kWarps + (int)(threadIdx.x >> 5),
                                                  fp32_dyn_smem);
 }
@@ -779,8 +780,7 @@ cudaError_t launch_t(const PivParams& p, cudaStream_t s)
         if (e != cudaSuccess) return e;
         attr_done[vec].fetch_or(bit);
     }
-    kern<<<(unsigned)blocks, 32 * kWarps, smem, s>>>(p);
-    return cudaGetLastError();
+    return launch_dependent(kern, (unsigned)blocks, 32 * kWarps, smem, s, p);
 }
 
 // frames (u8, u16, f32) without plane output; double windows (the per-window

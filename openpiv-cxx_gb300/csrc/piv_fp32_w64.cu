@@ -596,6 +596,7 @@ template <int MODE, bool LIMIT, typename PixT, bool PLANES>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 piv_w64_kernel(const PivParams p)
 {
+    after_previous();
     w64_task<MODE, LIMIT, PixT, PLANES>(p, (int)blockIdx.x);
 }
 
@@ -659,8 +660,7 @@ cudaError_t launch_t(const PivParams& p, cudaStream_t s)
         attr_done.fetch_or(bit);
     }
     const int64_t blocks = (p.n_win + 1) / 2;
-    piv_w64_kernel<MODE, LIMIT, PixT, PLANES><<<(unsigned)blocks, kThreads, smem, s>>>(p);
-    return cudaGetLastError();
+    return launch_dependent(piv_w64_kernel<MODE, LIMIT, PixT, PLANES>, (unsigned)blocks, kThreads, smem, s, p);
 }
 
 template <int MODE, bool LIMIT>

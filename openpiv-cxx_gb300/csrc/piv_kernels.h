@@ -64,6 +64,33 @@ struct alignas(16) PivParams {
 // are done; [2]: windows flagged in the last pass.
 constexpr int kFlagCounters = 3;
 
+// Programmatic dependent launch of a pass's kernels on one stream: the launch
+// is prepared while the kernel before it still runs, and the kernel calls
+// after_previous() before it touches memory, which waits for that kernel, and
+// with it all before it, to be complete.  Takes 3 to 4 us off the two launches
+// of a pass (160 x 128 px: 14.3 -> 10.8 us).  No kernel lets the next one's
+// blocks in early: it gained nothing (10.2 us there, 717 against 715 us for a
+// 4096 x 4096 pair) and waiting blocks hold room that other streams could use.
+template <typename... P, typename... A>
+inline cudaError_t launch_dependent(void (*kernel)(P...), unsigned int blocks, int threads, size_t smem,
+                                    cudaStream_t s, A&&... args)
+{
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3((unsigned int)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+#endif
+
 // Floats of a flagged window's record: the plane, its error bound, padding
 // to 16 bytes.
 __host__ __device__ constexpr int flag_record_floats(int w) { return w * w + 4; }
