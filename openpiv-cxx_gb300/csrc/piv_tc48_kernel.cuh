@@ -53,7 +53,15 @@ constexpr int kConstBytes = 2 * kSet;           // hi and lo parts (lo unused wi
 constexpr int kLo = 12288;                      // lo-part offset of the operand buffers
 constexpr int kPacked = 24576;                  // E2: k_x-slot-0 rows, 2 x 96 floats
 constexpr int kDataBytes = kPacked + 2 * 96 * 4;
-constexpr int kPS = W + 1;                      // E4 plane row stride (floats)
+// E4 plane: row stride (floats) and a column's place in a row.  A store's
+// lanes are 16 rows of both halves of a row: rows an odd multiple of 2 apart
+// fall on the even banks, and the odd shift of the second half puts it on the
+// odd ones (rows W + 1 apart and no shift: both halves on the same banks).
+// This and the scan's neighbours from the plane, split BF16 / FP16,
+// 2048 x 2048, step 12: 504 -> 455 us with both.
+constexpr int kPS = W + 2;
+__device__ __forceinline__ constexpr int plane_col(int x) { return x + (x >= H ? 1 : 0); }
+static_assert(kPS % 4 == 2 && H % 2 == 0, "plane banks");
 constexpr int kTailBytes = 1024;
 constexpr int kGroupBytes = (kDataBytes + kTailBytes + 1023) / 1024 * 1024;
 constexpr int kSmem = kConstBytes + kGroups * kGroupBytes;
@@ -670,7 +678,7 @@ piv_tc48_kernel(const PivParams p, const uint4* __restrict__ consts)
                     for (int i = 0; i < 24; ++i) v[i] *= us;
                 }
 #pragma unroll
-                for (int i = 0; i < 24; ++i) P[y * kPS + 24 * hh + i] = v[i];
+                for (int i = 0; i < 24; ++i) P[y * kPS + plane_col(H) * hh + i] = v[i];
                 if (p.planes) {
                     const int gw = grow * p.gnx + gcol;
 #pragma unroll
@@ -690,29 +698,26 @@ piv_tc48_kernel(const PivParams p, const uint4* __restrict__ consts)
 
         // ---- find_peaks: thread = (column x < 48 of 64, 24-row block); the
         // block's candidate rows roll through registers, neighbouring columns
-        // come from the neighbouring lanes (the two edge lanes of a warp read
-        // theirs); branch-free top two
+        // come from the plane (shuffles, with the edge lanes' own loads, took
+        // five shared-memory cycles a row where this takes three); branch-free
+        // top two
         {
             const int xs = tid & 63, yb = (tid >> 6) * 24;
             const bool col_ok = xs >= SX0 && xs < SX1;
             const int y0 = yb > SY0 ? yb : SY0, y1 = yb + 24 < SY1 ? yb + 24 : SY1;   // uniform over the warp
-            const int xl = xs == 0 ? W - 1 : xs - 1, xr = xs + 1 < W ? xs + 1 : 0;
             const int xc = xs < W ? xs : 0;   // columns 48..63 read column 0 (never candidates)
+            const int xl = xc == 0 ? W - 1 : xc - 1, xr = xc + 1 < W ? xc + 1 : 0;
             Top2 s{ TC_NEG_INF, TC_NEG_INF, 0x7fffffff };
-            float up = P[(y0 - 1) * kPS + xc], cc = P[y0 * kPS + xc];
+            const float *pc = P + plane_col(xc), *pl = P + plane_col(xl), *pr = P + plane_col(xr);
+            float up = pc[(y0 - 1) * kPS], cc = pc[y0 * kPS];
 #pragma unroll 4
             for (int ys = y0; ys < y1; ++ys) {
-                const float dn = P[(ys + 1) * kPS + xc];
-                const float sl = __shfl_up_sync(0xffffffffu, cc, 1);
-                const float sr = __shfl_down_sync(0xffffffffu, cc, 1);
-                const float lf = lane == 0 ? P[ys * kPS + xl] : sl;
-                const float rt = lane == 31 ? P[ys * kPS + xr] : sr;
+                const float dn = pc[(ys + 1) * kPS], lf = pl[ys * kPS], rt = pr[ys * kPS];
                 const float m = tcx::fmax3(up, dn, fmaxf(lf, rt));
                 const float sv = (col_ok && m < cc) ? cc : TC_NEG_INF;
-                const bool gt = sv > s.t0;
-                s.t1 = gt ? s.t0 : fmaxf(s.t1, sv);
-                s.key = gt ? ys * W + xs : s.key;
-                s.t0 = gt ? sv : s.t0;
+                s.t1 = fmaxf(s.t1, fminf(s.t0, sv));
+                s.key = sv > s.t0 ? ys * W + xs : s.key;
+                s.t0 = fmaxf(s.t0, sv);
                 up = cc;
                 cc = dn;
             }
@@ -749,8 +754,8 @@ piv_tc48_kernel(const PivParams p, const uint4* __restrict__ consts)
             const int ny = (j == 3 || j == 4) ? py - 1 : (j == 5 ? py + 1 : py);
             const int qx = (j == 0) ? px + 1 : px;
             const int qy = (j == 3) ? py + 1 : py;
-            const float an = P[ny * kPS + nx];
-            const float ad = P[qy * kPS + qx];
+            const float an = P[ny * kPS + plane_col(nx)];
+            const float ad = P[qy * kPS + plane_col(qx)];
             const float lg = log1pf((an - ad) / (ad + ped));
             const float lxr = __shfl_sync(0xffffffffu, lg, 0);
             const float lxl = __shfl_sync(0xffffffffu, lg, 1);
@@ -763,10 +768,11 @@ piv_tc48_kernel(const PivParams p, const uint4* __restrict__ consts)
                 opiv_vector out{ 0.f, 0.f, 0.f, 0.f, 0.f };
                 int32_t code = -1;
                 if (has2) {
-                    const float vc = P[py * kPS + px];
+                    const float* at = P + py * kPS;
+                    const float vc = at[plane_col(px)];
                     const float C = vc + ped;
-                    const float Lv = P[py * kPS + px - 1] + ped, R = P[py * kPS + px + 1] + ped;
-                    const float U = P[(py - 1) * kPS + px] + ped, D = P[(py + 1) * kPS + px] + ped;
+                    const float Lv = at[plane_col(px - 1)] + ped, R = at[plane_col(px + 1)] + ped;
+                    const float U = at[plane_col(px) - kPS] + ped, D = at[plane_col(px) + kPS] + ped;
                     const float nan = __int_as_float(0x7fffffff);
                     const bool okx = Lv > 0.f && C > 0.f && R > 0.f;
                     const bool oky = U > 0.f && C > 0.f && D > 0.f;

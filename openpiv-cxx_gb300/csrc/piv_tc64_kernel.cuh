@@ -61,7 +61,15 @@ constexpr int kConstBytes = 2 * kSet;           // hi and lo parts (lo unused wi
 constexpr int kDataBytes = 32768;               // stage-2 and stage-3 operands, hi and lo
 constexpr int kLo = 16384;                      // lo-part offset of the operand buffers
 constexpr int kPacked = 8192;                   // E2: k_x-slot-0 rows (in stage-3 operand rows 32..63)
-constexpr int kPS = W + 1;                      // E4 plane row stride (floats)
+// E4 plane: row stride (floats) and a column's place in a row.  A store's
+// lanes are 16 rows of both halves of a row: rows an odd multiple of 2 apart
+// fall on the even banks, and the odd shift of the second half puts it on the
+// odd ones (rows W + 1 apart and no shift: both halves on the same banks).
+// This and the scan's neighbours from the plane, split BF16 / FP16,
+// 2048 x 2048, step 16: 409 -> 344 us with both.
+constexpr int kPS = W + 2;
+__device__ __forceinline__ constexpr int plane_col(int x) { return x + (x >= H ? 1 : 0); }
+static_assert(kPS % 4 == 2 && H % 2 == 0, "plane banks");
 constexpr int kTailBytes = 1024;
 constexpr int kGroupBytes = kDataBytes + kTailBytes;
 constexpr int kSmem = kConstBytes + kGroups * kGroupBytes;
@@ -524,7 +532,7 @@ piv_tc64_kernel(const PivParams p, const uint4* __restrict__ consts)
                 for (int i = 0; i < 32; ++i) v[i] *= us;
             }
 #pragma unroll
-            for (int i = 0; i < 32; ++i) P[y * kPS + 32 * hh + i] = v[i];
+            for (int i = 0; i < 32; ++i) P[y * kPS + plane_col(H) * hh + i] = v[i];
             if (p.planes) {
                 const int gw = grow * p.gnx + gcol;
 #pragma unroll
@@ -543,28 +551,24 @@ piv_tc64_kernel(const PivParams p, const uint4* __restrict__ consts)
 
         // ---- find_peaks: thread = (column x, 32-row block); the block's
         // candidate rows roll through registers, neighbouring columns come
-        // from the neighbouring lanes (the two edge lanes of a warp read
-        // theirs); branch-free top two
+        // from the plane (shuffles, with the edge lanes' own loads, took five
+        // shared-memory cycles a row where this takes three); branch-free top two
         {
             const int xs = tid & 63, yb = (tid >> 6) * 32;
             const bool col_ok = xs >= SX0 && xs < SX1;
             const int y0 = yb > SY0 ? yb : SY0, y1 = yb + 32 < SY1 ? yb + 32 : SY1;   // uniform over the warp
             const int xl = (xs + W - 1) & (W - 1), xr = (xs + 1) & (W - 1);
             Top2 s{ TC_NEG_INF, TC_NEG_INF, 0x7fffffff };
-            float up = P[(y0 - 1) * kPS + xs], cc = P[y0 * kPS + xs];
+            const float *pc = P + plane_col(xs), *pl = P + plane_col(xl), *pr = P + plane_col(xr);
+            float up = pc[(y0 - 1) * kPS], cc = pc[y0 * kPS];
 #pragma unroll 4
             for (int ys = y0; ys < y1; ++ys) {
-                const float dn = P[(ys + 1) * kPS + xs];
-                const float sl = __shfl_up_sync(0xffffffffu, cc, 1);
-                const float sr = __shfl_down_sync(0xffffffffu, cc, 1);
-                const float lf = lane == 0 ? P[ys * kPS + xl] : sl;
-                const float rt = lane == 31 ? P[ys * kPS + xr] : sr;
+                const float dn = pc[(ys + 1) * kPS], lf = pl[ys * kPS], rt = pr[ys * kPS];
                 const float m = tcx::fmax3(up, dn, fmaxf(lf, rt));
                 const float sv = (col_ok && m < cc) ? cc : TC_NEG_INF;
-                const bool gt = sv > s.t0;
-                s.t1 = gt ? s.t0 : fmaxf(s.t1, sv);
-                s.key = gt ? ys * W + xs : s.key;
-                s.t0 = gt ? sv : s.t0;
+                s.t1 = fmaxf(s.t1, fminf(s.t0, sv));
+                s.key = sv > s.t0 ? ys * W + xs : s.key;
+                s.t0 = fmaxf(s.t0, sv);
                 up = cc;
                 cc = dn;
             }
@@ -601,8 +605,8 @@ piv_tc64_kernel(const PivParams p, const uint4* __restrict__ consts)
             const int ny = (j == 3 || j == 4) ? py - 1 : (j == 5 ? py + 1 : py);
             const int qx = (j == 0) ? px + 1 : px;
             const int qy = (j == 3) ? py + 1 : py;
-            const float an = P[(ny & (W - 1)) * kPS + (nx & (W - 1))];
-            const float ad = P[(qy & (W - 1)) * kPS + (qx & (W - 1))];
+            const float an = P[(ny & (W - 1)) * kPS + plane_col(nx & (W - 1))];
+            const float ad = P[(qy & (W - 1)) * kPS + plane_col(qx & (W - 1))];
             const float lg = log1pf((an - ad) / (ad + ped));
             const float lxr = __shfl_sync(0xffffffffu, lg, 0);
             const float lxl = __shfl_sync(0xffffffffu, lg, 1);
@@ -615,10 +619,11 @@ piv_tc64_kernel(const PivParams p, const uint4* __restrict__ consts)
                 opiv_vector out{ 0.f, 0.f, 0.f, 0.f, 0.f };
                 int32_t code = -1;
                 if (has2) {
-                    const float vc = P[py * kPS + px];
+                    const float* at = P + py * kPS;
+                    const float vc = at[plane_col(px)];
                     const float C = vc + ped;
-                    const float Lv = P[py * kPS + px - 1] + ped, R = P[py * kPS + px + 1] + ped;
-                    const float U = P[(py - 1) * kPS + px] + ped, D = P[(py + 1) * kPS + px] + ped;
+                    const float Lv = at[plane_col(px - 1)] + ped, R = at[plane_col(px + 1)] + ped;
+                    const float U = at[plane_col(px) - kPS] + ped, D = at[plane_col(px) + kPS] + ped;
                     const float nan = __int_as_float(0x7fffffff);
                     const bool okx = Lv > 0.f && C > 0.f && R > 0.f;
                     const bool oky = U > 0.f && C > 0.f && D > 0.f;
