@@ -295,6 +295,7 @@ piv_tc48_kernel(const PivParams p, const uint4* __restrict__ consts)
     constexpr uint32_t kId4 = tcx::idesc_f16kind(64, 48, false, F16);
 
     extern __shared__ __align__(1024) unsigned char smem[];
+    after_previous();
     unsigned char* cst = smem;
     const int grp = (int)(threadIdx.x / kThreads);
     unsigned char* dat = smem + kConstBytes + grp * kGroupBytes;
@@ -831,8 +832,7 @@ cudaError_t launch_t(const PivParams& p, const void* consts, cudaStream_t s)
     const int64_t want = (p.n_win + kGroups - 1) / kGroups;
     const int blocks = (int)(want < cap ? want : cap);
     if (blocks <= 0) return cudaSuccess;
-    kern<<<blocks, kThreads * kGroups, kSmem, s>>>(p, reinterpret_cast<const uint4*>(consts));
-    return cudaGetLastError();
+    return launch_dependent(kern, (unsigned int)blocks, kThreads * kGroups, kSmem, s, p, reinterpret_cast<const uint4*>(consts));
 }
 
 template <bool F16, bool SPLIT, bool CSPLIT, int MODE, bool LIMIT>

@@ -281,6 +281,7 @@ piv_tc_kernel(const PivParams p, const uint4* __restrict__ consts)
     constexpr uint32_t kIdM64 = tcx::idesc_f16kind(128, 64, true, F16);
 
     extern __shared__ __align__(1024) unsigned char smem[];
+    after_previous();
     unsigned char* cst = smem;
     // this thread's tile group: its data buffer and tail
     const int grp = GROUPS == 1 ? 0 : (int)(threadIdx.x / kThreads);
@@ -926,8 +927,7 @@ cudaError_t launch_t(const PivParams& p, const void* consts, cudaStream_t s)
     const int64_t want = (tiles + G - 1) / G;
     const int blocks = (int)(want < cap ? want : cap);
     if (blocks <= 0) return cudaSuccess;
-    kern<<<blocks, kThreads * G, kSmem, s>>>(p, reinterpret_cast<const uint4*>(consts));
-    return cudaGetLastError();
+    return launch_dependent(kern, (unsigned int)blocks, kThreads * G, kSmem, s, p, reinterpret_cast<const uint4*>(consts));
 }
 
 template <bool F16, bool SPLIT, bool CSPLIT, int MODE, bool LIMIT>

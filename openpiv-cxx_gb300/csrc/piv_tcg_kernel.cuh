@@ -165,6 +165,7 @@ piv_tcg_kernel(const PivParams p, const uint4* __restrict__ consts, int mode, in
     const int SY0 = D0 + 1, SY1 = D0 + VW - 2, SX0 = D0 + 1, SX1 = D0 + VW - 1;
 
     extern __shared__ __align__(1024) unsigned char smem[];
+    after_previous();
     unsigned char* cst = smem;
     unsigned char* dat = smem + G::kCParts * G::kSet;
     float* xch = reinterpret_cast<float*>(dat + G::kParts * G::kOp);   // exchange rows, then planes
@@ -610,8 +611,7 @@ cudaError_t launch_t(const PivParams& p, int mode, int limit, const void* consts
     const int64_t c = cap[dev & 63].load();
     const int blocks = (int)(tiles < c ? tiles : c);
     if (blocks <= 0) return cudaSuccess;
-    kern<<<blocks, kThreads, G::kSmem, s>>>(p, reinterpret_cast<const uint4*>(consts), mode, limit);
-    return cudaGetLastError();
+    return launch_dependent(kern, (unsigned int)blocks, kThreads, G::kSmem, s, p, reinterpret_cast<const uint4*>(consts), mode, limit);
 }
 
 // one window size: operand type, MMAs per product (3: data and constants
