@@ -274,8 +274,8 @@ class Plan:
                                 f"image size is different from expected: {f.shape} {f.dtype}")
         fa = np.ascontiguousarray(frame_a)
         fb = np.ascontiguousarray(frame_b)
-        vec = np.zeros((self.n, 5), np.float32)
-        pk = np.zeros(self.n, np.int32) if with_peaks else None
+        vec = np.empty((self.n, 5), np.float32)
+        pk = np.empty(self.n, np.int32) if with_peaks else None
         _check(load().opiv_process_pair(self._h, fa.ctypes.data, fb.ctypes.data, fa.strides[0],
                                         vec.ctypes.data, pk.ctypes.data if with_peaks else None))
         return vec, pk
@@ -362,9 +362,9 @@ class Plan:
 # ---- multi-pass window offsetting ------------------------------------------
 def unpack_disp(d: np.ndarray) -> np.ndarray:
     """(n,) packed (dy << 16) | (dx & 0xffff) -> (n, 2) int (dx, dy)."""
-    d = np.asarray(d, np.int32)
-    return np.stack([(d & 0xFFFF).astype(np.uint16).astype(np.int16).astype(np.int64),
-                     (d >> 16).astype(np.int64)], 1)
+    d = np.ascontiguousarray(d, np.int32)
+    # the halves of a little-endian word: dx first (one pass instead of five)
+    return d.view(np.int16).reshape(-1, 2).astype(np.int64)
 
 
 class MultiPass:
@@ -408,18 +408,18 @@ class MultiPass:
         fa = np.ascontiguousarray(frame_a, self.dtype)
         fb = np.ascontiguousarray(frame_b, self.dtype)
         n = self.counts[-1]
-        vec = np.zeros((n, 5), np.float32)
-        pk = np.zeros(n, np.int32)
-        disp = np.zeros(n, np.int32)
+        vec = np.empty((n, 5), np.float32)
+        pk = np.empty(n, np.int32)
+        disp = np.empty(n, np.int32)
         _check(load().opiv_multipass_process(self._h, fa.ctypes.data, fb.ctypes.data, fa.strides[0],
                                              vec.ctypes.data, pk.ctypes.data, disp.ctypes.data))
         return vec, pk, unpack_disp(disp)
 
     def results(self, k: int):
         n = self.counts[k]
-        vec = np.zeros((n, 5), np.float32)
-        pk = np.zeros(n, np.int32)
-        disp = np.zeros(n, np.int32)
+        vec = np.empty((n, 5), np.float32)
+        pk = np.empty(n, np.int32)
+        disp = np.empty(n, np.int32)
         _check(load().opiv_multipass_results(self._h, k, vec.ctypes.data, pk.ctypes.data,
                                              disp.ctypes.data))
         return vec, pk, unpack_disp(disp)
@@ -520,9 +520,9 @@ class Batch:
 
     def results(self, pair: int, k: int):
         n = self.window_count(pair, k)
-        vec = np.zeros((n, 5), np.float32)
-        pk = np.zeros(n, np.int32)
-        disp = np.zeros(n, np.int32)
+        vec = np.empty((n, 5), np.float32)
+        pk = np.empty(n, np.int32)
+        disp = np.empty(n, np.int32)
         _check(load().opiv_batch_results(self._h, pair, k, vec.ctypes.data, pk.ctypes.data,
                                          disp.ctypes.data))
         return vec, pk, unpack_disp(disp)
