@@ -70,10 +70,10 @@ L2_ROTATION = 4
 # SHA-256 prefixes of the kernel sources that capture ran: when a source no
 # longer matches, the line reports no traffic instead of a stale figure
 KERNEL_TRAFFIC = {
-    "tc": {"bytes": 67_346_944 + 819_456,
-           "sources": {"piv_tc_kernel.cuh": "52baeb2ef1e34e1b", "tc_ptx.cuh": "74cf252d23d6309a"}},
-    "fp32": {"bytes": 67_165_440 + 4_344_832,
-             "sources": {"piv_fp32.cuh": "916731b6afc83819", "fft_reg.cuh": "b328bf1c452ce151"}},
+    "tc": {"bytes": 67_309_056 + 95_744,
+           "sources": {"piv_tc_kernel.cuh": "e89e8fd5118876f1", "tc_ptx.cuh": "74cf252d23d6309a"}},
+    "fp32": {"bytes": 67_160_576 + 4_210_176,
+             "sources": {"piv_fp32.cuh": "bf57c59dd05ec6c9", "fft_reg.cuh": "59d479598caf2c38"}},
 }
 
 
@@ -875,6 +875,11 @@ def adjoint_line(mc_seeds):
     ga = torch.zeros_like(da)
     gb = torch.zeros_like(db)
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    # the first call of a kernel loads it: not timed
+    plan.adjoint_device(da.data_ptr(), db.data_ptr(), pitch, pk.data_ptr(), cot.data_ptr(),
+                        ga.data_ptr(), gb.data_ptr(), pitch)
+    ga.zero_()
+    gb.zero_()
     ev0.record()
     plan.adjoint_device(da.data_ptr(), db.data_ptr(), pitch, pk.data_ptr(), cot.data_ptr(),
                         ga.data_ptr(), gb.data_ptr(), pitch)
@@ -907,6 +912,8 @@ def adjoint_line(mc_seeds):
     c0a, c0b = torch.from_numpy(a0).cuda(), torch.from_numpy(b0).cuda()
     plan.process_device(c0a.data_ptr(), c0b.data_ptr(), pitch, vec.data_ptr(), pk.data_ptr(), 0)
     dsig = torch.zeros((plan.n, 2), dtype=torch.float32, device="cuda")
+    plan.adjoint_device(c0a.data_ptr(), c0b.data_ptr(), pitch, pk.data_ptr(), var_a=sig * sig,
+                        var_b=sig * sig, d_sigma=dsig.data_ptr())   # the first call loads the kernel
     ev0.record()
     plan.adjoint_device(c0a.data_ptr(), c0b.data_ptr(), pitch, pk.data_ptr(), var_a=sig * sig,
                         var_b=sig * sig, d_sigma=dsig.data_ptr())

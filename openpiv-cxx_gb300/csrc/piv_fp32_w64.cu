@@ -35,10 +35,10 @@
 // 2048 x 2048, u16, step 16 (15,625 windows): 464 us with two tiles, seventeen
 // trips through shared memory and a serial fit on one thread, 240 us with
 // this (13,300 warp instructions a window where it took 21,600).  Packed FP32
-// (add2, sub2, fma2) took 268 to 242 us of that: the kernel is bound by issue
-// slots (about 75 % busy), then by shared-memory wavefronts (65 %), so one
-// instruction for both components pays although the FP32 pipe's rate is the
-// same.  One tile (33 KB) and 64 registers let four CTAs share an SM.
+// (add2, sub2, fma2) took 268 to 242 us of that: issue slots are 70 % busy
+// (L1 and shared memory 81 %), so one instruction for both components pays
+// although the FP32 pipe's rate is the same.  One tile (33 KB) and 64
+// registers let four CTAs share an SM.
 
 #include <atomic>
 #include <cstdint>
