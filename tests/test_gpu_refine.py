@@ -26,7 +26,7 @@ def frames(kind, dtype, h, w, seed):
     texture = (texture + np.roll(texture, 1, 0) + np.roll(texture, 1, 1) + np.roll(texture, (1, 1), (0, 1))) / 2
     a, b = texture[3:3 + h, 5:5 + w], texture[5:5 + h, 4:4 + w]
     if kind == "two_level":
-        top = 255 if dtype == np.uint8 else 1
+        top = 1 if dtype == np.float32 else 255
         return tuple((f > 1.5).astype(dtype) * dtype(top) for f in (a, b))
     level, spread = {np.uint8: (200, 3), np.uint16: (4000, 200), np.float32: (3.0, 0.1)}[dtype]
     pair = [level + spread * f + spread * rng.normal(0.0, 0.5, f.shape) for f in (a, b)]
@@ -61,3 +61,33 @@ def test_flagged_windows_against_oracle(orc, kind, dtype, limit, ia, mode):
     d = np.abs(got - want)
     assert np.nanmax(d[:, 2:4], initial=0.0) <= 3e-6
     assert np.nanmax(d[:, 4] / np.maximum(np.abs(want[:, 4]), 1e-30), initial=0.0) <= 1e-6
+
+
+@pytest.mark.parametrize("ia", [16, 32, 64])
+def test_counters_between_passes(ia):
+    """The second launch leaves the flag counters ready: passes over frames
+    that flag many windows, few and many again on one plan, and the pipelined
+    call over both, give what a fresh plan gives."""
+    h, w = 3 * ia + 7, 4 * ia + 9
+    many = frames("pedestal", np.uint16, h, w, 11)
+    few = frames("two_level", np.uint16, h, w, 12)
+
+    def fresh(pair):
+        plan = og.Plan(w, h, np.uint16, ia, ia // 2, ia // 4 + 1)
+        out = plan.process(*pair), plan.exact_count()
+        plan.close()
+        return out
+
+    want = {id(p): fresh(p) for p in (many, few)}
+    assert want[id(many)][1] != want[id(few)][1]
+    plan = og.Plan(w, h, np.uint16, ia, ia // 2, ia // 4 + 1)
+    order = (many, few, many, many, few)
+    for pair in order:
+        (vec, pk), n = plan.process(*pair), plan.exact_count()
+        ref, count = want[id(pair)]
+        assert n == count
+        assert np.array_equal(vec, ref[0], equal_nan=True) and np.array_equal(pk, ref[1])
+    for (vec, pk), pair in zip(plan.process_pairs(list(order)), order):
+        ref = want[id(pair)][0]
+        assert np.array_equal(vec, ref[0], equal_nan=True) and np.array_equal(pk, ref[1])
+    plan.close()
