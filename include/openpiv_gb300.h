@@ -121,9 +121,12 @@ int opiv_process_pair_device(opiv_plan* plan, const void* d_frame_a, const void*
                              size_t pitch_bytes, opiv_vector* d_out_vec, int32_t* d_out_peak,
                              void* stream);
 
-/* number of windows the last pass sent to the exact double-precision
- * re-evaluation (synchronises with the plan's last pass) */
+/* number of windows the last pass sent to the exact re-evaluation
+ * (synchronises with the plan's last pass), and how many of those were
+ * decided from exact correlation sums; the others took the reference's
+ * double arithmetic */
 int64_t opiv_plan_exact_count(opiv_plan* plan);
+int64_t opiv_plan_settled_count(opiv_plan* plan);
 
 /* Many image pairs of the plan's size through opiv_process_pair's pass,
  * pipelined: the upload of pair i+1 and the download of pair i-1 overlap

@@ -738,7 +738,10 @@ int opiv_process_pairs(opiv_plan* plan, int64_t n_pairs, const void* const* fram
     return done(OPIV_OK);
 }
 
-int64_t opiv_plan_exact_count(opiv_plan* plan)
+namespace {
+
+// Counter `at` of the plan's last pass.
+int64_t last_flag_counter(opiv_plan* plan, int at)
 {
     if (!plan) return fail(OPIV_ERR_ARG, "plan is null");
     unsigned int count = 0;
@@ -747,11 +750,16 @@ int64_t opiv_plan_exact_count(opiv_plan* plan)
     cudaGetDevice(&prev);
     cudaSetDevice(plan->device);
     cudaDeviceSynchronize();
-    const cudaError_t e = cudaMemcpy(&count, plan->d_flag_count + 2, sizeof count, cudaMemcpyDeviceToHost);
+    const cudaError_t e = cudaMemcpy(&count, plan->d_flag_count + at, sizeof count, cudaMemcpyDeviceToHost);
     cudaSetDevice(prev);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpy(flag count)");
     return (int64_t)count;
 }
+
+}  // namespace
+
+int64_t opiv_plan_exact_count(opiv_plan* plan) { return last_flag_counter(plan, 2); }
+int64_t opiv_plan_settled_count(opiv_plan* plan) { return last_flag_counter(plan, 4); }
 
 int opiv_multipass_create(opiv_multipass** out, uint32_t img_w, uint32_t img_h, int dtype,
                           int n_passes, const uint32_t* ia, const uint32_t* step, int mode,

@@ -61,8 +61,9 @@ struct alignas(16) PivParams {
 };
 
 // flag_count[0]: windows flagged so far; [1]: CTAs of the exact launch that
-// are done; [2]: windows flagged in the last pass.
-constexpr int kFlagCounters = 3;
+// are done; [2]: windows flagged in the last pass; [3]: flagged windows decided
+// from exact sums so far; [4]: in the last pass.
+constexpr int kFlagCounters = 5;
 
 // Programmatic dependent launch of a pass's kernels on one stream: the launch
 // is prepared while the kernel before it still runs, and the kernel calls

@@ -46,7 +46,8 @@ SYMBOLS = [
     "opiv_last_error", "opiv_status_string", "opiv_version", "opiv_kernel_launch_count",
     "opiv_grid", "opiv_grid_offsets", "opiv_plan_create", "opiv_plan_destroy",
     "opiv_plan_window_count", "opiv_plan_grid", "opiv_process_pair",
-    "opiv_process_pair_device", "opiv_plan_exact_count", "opiv_plan_set_timing",
+    "opiv_process_pair_device", "opiv_plan_exact_count", "opiv_plan_settled_count",
+    "opiv_plan_set_timing",
     "opiv_plan_last_timing", "opiv_cross_correlate_batch",
     "opiv_find_peaks", "opiv_fit_simple_gaussian", "opiv_process_pair_device_noalloc",
     "opiv_transform_batch", "opiv_transform_real_batch", "opiv_auto_correlate_batch",
@@ -118,6 +119,8 @@ def load(path: str | None = None) -> C.CDLL:
                                            C.c_void_p, C.c_void_p, C.c_void_p]
     L.opiv_plan_exact_count.restype = C.c_int64
     L.opiv_plan_exact_count.argtypes = [C.c_void_p]
+    L.opiv_plan_settled_count.restype = C.c_int64
+    L.opiv_plan_settled_count.argtypes = [C.c_void_p]
     L.opiv_plan_set_timing.argtypes = [C.c_void_p, C.c_int]
     L.opiv_plan_set_precision.argtypes = [C.c_void_p, C.c_int]
     L.opiv_plan_set_tile.argtypes = [C.c_void_p, C.c_int]
@@ -292,6 +295,9 @@ class Plan:
 
     def exact_count(self) -> int:
         return int(load().opiv_plan_exact_count(self._h))
+
+    def settled_count(self) -> int:
+        return int(load().opiv_plan_settled_count(self._h))
 
     def process_pairs_into(self, ptrs_a, ptrs_b, pitch: int, ptrs_vec, ptrs_peak=None):
         """Host pointers (pinned for overlap), one per pair: pipelined passes."""
