@@ -71,6 +71,15 @@ constexpr int kWarps = 4;   // warps per CTA
 constexpr float kFitTol = 6e-5f;
 constexpr float kSnTol = 6e-6f;
 constexpr float kSnCap = 4.f;
+// A window whose lanes' energies (`lanes` of them) stay below this overflows
+// nowhere: plane and spectrum values are at most 8 W^2 times its energy.
+// Beyond, and where a pixel is NaN, the pair is transformed without it (one
+// transform carries both planes, so it would take the other window with it):
+// with a NaN pixel every plane value is NaN and there is no peak; otherwise
+// FP64 decides.  The per-window planes (double windows) only ask for finite.
+template <bool PLANES>
+__host__ __device__ constexpr float max_energy(int w, int lanes) { return PLANES ? 3.4e38f : 3e38f / (8.f * (float)(w * w) * (float)lanes); }
+enum { kBadHuge = 1, kBadNan = 2 };
 #define kNegInf (-__int_as_float(0x7f800000))
 constexpr float kTwo23 = 8388608.0f;
 
@@ -409,6 +418,7 @@ __device__ __forceinline__ void fp32_task(const PivParams& p, const int task, fl
     float2 v[W];      // the transform being worked on
     float2 energy = make_float2(0.f, 0.f);
     float ped0 = 0.f, ped1 = 0.f;
+    int bad = 0;      // float windows: kBad bits, the second window's two up
 
 #pragma unroll 1
     for (int st = 0; st < 6; ++st) {
@@ -447,8 +457,23 @@ __device__ __forceinline__ void fp32_task(const PivParams& p, const int task, fl
                 else
                     load_window<W, true, true, PixT>(ca, cb, pitch, gl, tile, v);
             }
+            const float2 before = energy;
 #pragma unroll
             for (int x = 0; x < W; ++x) energy = fma2(v[x], v[x], energy);
+            if constexpr (sizeof(PixT) >= 4) {
+                const float e = energy.x + energy.y;
+                const unsigned over = __ballot_sync(0xffffffffu, !(e < max_energy<PLANES>(W, W)));
+                if (over != 0) {
+                    const unsigned nan = __ballot_sync(0xffffffffu, e != e);
+                    const unsigned mine = (W == 32 ? 0xffffffffu : (1u << W) - 1u) << (grp * W % 32);
+                    if (over & mine) {
+                        bad |= ((nan & mine) ? kBadNan : kBadHuge) << (2 * h);
+                        energy = before;
+#pragma unroll
+                        for (int x = 0; x < W; ++x) v[x] = make_float2(0.f, 0.f);
+                    }
+                }
+            }
         } else if (st == kStCol0 || st == kStCol1) {
             // v: lane = y, register kx.  Transpose to lane = kx, register
             // bitrev(y).  REAL mode: column kx = 0 of Z is zeroed here, so
@@ -536,7 +561,8 @@ __device__ __forceinline__ void fp32_task(const PivParams& p, const int task, fl
             if (w >= (int)p.n_win) continue;
             for (int y = 0; y < W; ++y) {
                 const float2 c = S[tix<W>(y, gl)];   // the lane's own column
-                p.planes[(size_t)w * N + ((y + W / 2) & (W - 1)) * W + xs] = 0.25f * (h ? c.y : c.x);
+                p.planes[(size_t)w * N + ((y + W / 2) & (W - 1)) * W + xs] =
+                    (bad >> (2 * h)) & 3 ? __int_as_float(0x7fffffff) : 0.25f * (h ? c.y : c.x);
             }
         }
     }
@@ -600,7 +626,8 @@ __device__ __forceinline__ void fp32_task(const PivParams& p, const int task, fl
 #pragma unroll
     for (int o = HL / 2; o > 0; o >>= 1) g.merge(g.across(o));
 
-    const bool has2 = g.t1 > kNegInf;
+    const int bad_h = (bad >> (2 * h)) & 3;
+    const bool has2 = bad_h == 0 && g.t1 > kNegInf;
     const int px = has2 ? g.key % W : HL, py = has2 ? g.key / W : HL;       // swapped-plane coordinates
     const int ux = (px + W / 2) & (W - 1), uy = (py + W / 2) & (W - 1);
     const float ped = h ? ped1 : ped0;
@@ -632,7 +659,9 @@ __device__ __forceinline__ void fp32_task(const PivParams& p, const int task, fl
         int bx, by, ox, oy;
         window_origin(p, w, bx, by);
         b_offset(p, W, bx, by, ox, oy);
-        if (!has2) {
+        if (bad_h != 0) {
+            certain = bad_h == kBadNan;
+        } else if (!has2) {
             certain = !(g.umax > kNegInf);
         } else {
             const float C = vc + ped, L = vl + ped, R = vr + ped, U = vu + ped, D = vd + ped;
@@ -683,7 +712,7 @@ __device__ __forceinline__ void fp32_task(const PivParams& p, const int task, fl
         float* rec = p.flag_planes + (size_t)slot * flag_record_floats(W);
 #pragma unroll 1
         for (int i = hl; i < N; i += HL) rec[i] = cell(i / W + W / 2, i % W + W / 2);
-        if (hl == 0) rec[N] = dlt;
+        if (hl == 0) rec[N] = bad_h == 0 ? dlt : 0.f;   // without a bound: to the FP64 transforms
     }
 }
 

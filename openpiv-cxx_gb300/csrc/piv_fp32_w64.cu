@@ -61,6 +61,10 @@ constexpr int kCtasPerSm = 4;
 constexpr float kFitTol = 6e-5f;
 constexpr float kSnTol = 6e-6f;
 constexpr float kSnCap = 4.f;
+// windows with pixels that are not finite, or too large: as there
+template <bool PLANES>
+__host__ __device__ constexpr float max_energy() { return PLANES ? 3.4e38f : 3e38f / (8.f * (float)N * (float)kThreads); }
+enum { kBadHuge = 1, kBadNan = 2 };
 #define kNegInf64 (-__int_as_float(0x7f800000))
 
 // base-8 digit reversal of a 6-bit index (an involution)
@@ -346,6 +350,7 @@ __device__ __forceinline__ void w64_task(const PivParams& p, const int blk)
     float2* const eb = T + 8 * jb * LD + cb;
 
     float2 energy = make_float2(0.f, 0.f);
+    int bad = 0;      // float windows: kBad bits, the second window's two up
     pair_slot first[8];
 #pragma unroll 1
     for (int h = 0; h < 2; ++h) {
@@ -359,6 +364,7 @@ __device__ __forceinline__ void w64_task(const PivParams& p, const int blk)
             const PixT* fa = reinterpret_cast<const PixT*>(p.fa) + (size_t)by * pitch + bx + x;
             const PixT* fb = reinterpret_cast<const PixT*>(p.fb) + (size_t)(by + oy) * pitch + bx + ox + x;
             double sa = 0.0, sb = 0.0;
+            const float2 before = energy;
 #pragma unroll
             for (int it = 0; it < 2; ++it) {
                 const int j1 = (t >> 6) + 4 * it;   // rows j1 + 8 m of column x
@@ -400,7 +406,17 @@ __device__ __forceinline__ void w64_task(const PivParams& p, const int blk)
                     p.peds[w0 + h] = (MODE == kModeComplex) ? sa * sb : 0.0;
                 }
             }
-            __syncthreads();
+            if constexpr (sizeof(PixT) >= 4) {
+                const float e = energy.x + energy.y;
+                if (__syncthreads_or(!(e < max_energy<PLANES>()))) {
+                    bad |= (__syncthreads_or(e != e) ? kBadNan : kBadHuge) << (2 * h);
+                    energy = before;
+                    for (int i = t >> 6; i < W; i += kThreads / W) T[x * LD + i] = make_float2(0.f, 0.f);
+                    __syncthreads();
+                }
+            } else {
+                __syncthreads();
+            }
             pass8<true, true, false>(T, tw);
             pass8<false, false, true>(T, tw);
             load8<LD>(ea, A);
@@ -467,7 +483,8 @@ __device__ __forceinline__ void w64_task(const PivParams& p, const int blk)
         for (int h = 0; h < (valid1 ? 2 : 1); ++h)
             for (int i = t; i < N; i += kThreads) {
                 const float2 v = cell(i >> 6, i & 63);
-                p.planes[(size_t)(w0 + h) * N + i] = 0.25f * (h ? v.y : v.x);
+                p.planes[(size_t)(w0 + h) * N + i] =
+                    (bad >> (2 * h)) & 3 ? __int_as_float(0x7fffffff) : 0.25f * (h ? v.y : v.x);
             }
 
     // ---- find_peaks on both planes at once: thread = (column, 16-row
@@ -523,7 +540,8 @@ __device__ __forceinline__ void w64_task(const PivParams& p, const int blk)
             const float2 v = cell(ys, xs);
             return h ? v.y : v.x;
         };
-        const bool has2 = g.t1 > kNegInf64;
+        const int bad_h = (bad >> (2 * h)) & 3;
+        const bool has2 = bad_h == 0 && g.t1 > kNegInf64;
         const int px = has2 ? g.key % W : W / 2, py = has2 ? g.key / W : W / 2;
         const float vc = val(py, px), vl = val(py, px - 1), vr = val(py, px + 1);
         const float vu = val(py - 1, px), vd = val(py + 1, px);
@@ -544,7 +562,9 @@ __device__ __forceinline__ void w64_task(const PivParams& p, const int blk)
             opiv_vector out{ 0.f, 0.f, 0.f, 0.f, 0.f };
             int32_t code = -1;
             bool certain;
-            if (!has2) {
+            if (bad_h != 0) {
+                certain = bad_h == kBadNan;
+            } else if (!has2) {
                 certain = !(g.umax > kNegInf64);
             } else {
                 const float C = vc + ped, L = vl + ped, R = vr + ped, U = vu + ped, D = vd + ped;
@@ -587,7 +607,7 @@ __device__ __forceinline__ void w64_task(const PivParams& p, const int blk)
         if (!PLANES && slot >= 0) {
             float* rec = p.flag_planes + (size_t)slot * flag_record_floats(W);
             for (int i = lane; i < N; i += 32) rec[i] = val(i >> 6, i & 63);
-            if (lane == 0) rec[N] = dlt;
+            if (lane == 0) rec[N] = bad_h == 0 ? dlt : 0.f;   // without a bound: to the FP64 transforms
         }
     }
 }
