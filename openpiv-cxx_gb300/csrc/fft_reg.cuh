@@ -110,13 +110,6 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b)
     return d;
 }
 
-__device__ __forceinline__ float2 mul2(float2 a, float2 b)
-{
-    float2 d;
-    asm("{ .reg .b64 x, y; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; mul.rn.f32x2 x, x, y; mov.b64 {%0, %1}, x; }"
-        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return d;
-}
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
 {
     float2 d;

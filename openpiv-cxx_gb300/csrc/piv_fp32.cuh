@@ -48,39 +48,13 @@
 
 #include "fft_reg.cuh"
 #include "offsets.cuh"
+#include "peak_scan.cuh"
 #include "piv_kernels.h"
 
 namespace opiv {
 namespace fp32 {
 
 constexpr int kWarps = 4;   // warps per CTA
-// A window is decided by this kernel only if the error bound of its
-// sub-pixel fit stays below kFitTol pixels and the relative error bound of
-// its sn below kSnTol * (1 + sn).  The parity tolerances are 1e-4 px and
-// 1e-5 * (1 + sn): sn = p0 / p1 is a ratio of plane values, and plane values
-// are specified to 1e-5 of the plane peak p0, which bounds the relative
-// error of p1 by 1e-5 * p0 / p1 = 1e-5 * sn.  The thresholds sit 1.6x inside
-// those tolerances (the rounding of the final FP32 logarithms, sums and
-// ratio adds ~1e-6 px and ~2e-7 relative on top of the bounds).  At 3e-5 /
-// 3e-6 three times as many 16 px windows went to the exact pass, nearly all
-// of them for the sn bound.  The factor 1 + sn ends at kSnCap: a few windows
-// of sn in the tens, whose second peak is little more than rounding, carried
-// nearly all of a field's sn error (2048 x 1536 field of 16 px windows: 1e-6 of
-// its norm, 1e-7 with the cap, 139 windows flagged where 78 were; REAL mode
-// with the limited search up to 1.5e-3 and 4e-8).
-constexpr float kFitTol = 6e-5f;
-constexpr float kSnTol = 6e-6f;
-constexpr float kSnCap = 4.f;
-// A window whose lanes' energies (`lanes` of them) stay below this overflows
-// nowhere: plane and spectrum values are at most 8 W^2 times its energy.
-// Beyond, and where a pixel is NaN, the pair is transformed without it (one
-// transform carries both planes, so it would take the other window with it):
-// with a NaN pixel every plane value is NaN and there is no peak; otherwise
-// FP64 decides.  The per-window planes (double windows) only ask for finite.
-template <bool PLANES>
-__host__ __device__ constexpr float max_energy(int w, int lanes) { return PLANES ? 3.4e38f : 3e38f / (8.f * (float)(w * w) * (float)lanes); }
-enum { kBadHuge = 1, kBadNan = 2 };
-#define kNegInf (-__int_as_float(0x7f800000))
 constexpr float kTwo23 = 8388608.0f;
 
 // ---- pixel loading -----------------------------------------------------------
@@ -337,53 +311,6 @@ __device__ __forceinline__ int tix(int r, int c) { return r * (W + 1) + c; }
 // shared memory per lane group: transpose tile + half spectrum
 template <int W>
 __host__ __device__ constexpr int group_smem_float2() { return W * (W + 1) + W * (W / 2 + 1); }
-
-// Running top-2 of strict 4-neighbour maxima (find_peaks) plus the largest
-// value whose strict-maximum decision is within dlt of flipping.
-struct Top2 {
-    float t0, t1, umax;
-    int key;
-    __device__ __forceinline__ void init()
-    {
-        t0 = t1 = umax = kNegInf;
-        key = 0;
-    }
-    __device__ __forceinline__ void add(float c, float m, float dlt, int k)
-    {
-        const float dd = m - c;
-        umax = fabsf(dd) <= dlt ? fmaxf(umax, c) : umax;
-        const float v = dd < 0.f ? c : kNegInf;
-        t1 = fmaxf(t1, fminf(t0, v));
-        key = v > t0 ? k : key;
-        t0 = fmaxf(t0, v);
-    }
-    // with another's (ties to the lowest row-major index)
-    __device__ __forceinline__ void merge(const Top2& o)
-    {
-        const bool take = (o.t0 > t0) || (o.t0 == t0 && o.key < key);
-        t1 = fmaxf(fmaxf(t1, o.t1), fminf(t0, o.t0));
-        key = take ? o.key : key;
-        t0 = fmaxf(t0, o.t0);
-        umax = fmaxf(umax, o.umax);
-    }
-    __device__ __forceinline__ Top2 across(int o) const   // the lane o away
-    {
-        Top2 r;
-        r.t0 = __shfl_xor_sync(0xffffffffu, t0, o);
-        r.t1 = __shfl_xor_sync(0xffffffffu, t1, o);
-        r.umax = __shfl_xor_sync(0xffffffffu, umax, o);
-        r.key = __shfl_xor_sync(0xffffffffu, key, o);
-        return r;
-    }
-};
-
-// a three-source max and a max
-__device__ __forceinline__ float max4(float a, float b, float c, float d)
-{
-    float m;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(fmaxf(c, d)));
-    return m;
-}
 
 // Transform stages of a pair, run by one runtime loop around one FFT body.
 enum { kStLoad0 = 0, kStCol0 = 1, kStLoad1 = 2, kStCol1 = 3, kStInvA = 4, kStInvB = 5 };

@@ -46,6 +46,7 @@
 
 #include "fft_reg.cuh"
 #include "offsets.cuh"
+#include "peak_scan.cuh"
 #include "piv_kernels.h"
 
 namespace opiv {
@@ -57,15 +58,6 @@ constexpr int LD = W + 1;            // row stride (float2), odd: rows fall on d
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kCtasPerSm = 4;
-// certification thresholds: as the 16 / 32 px kernel (piv_fp32.cuh)
-constexpr float kFitTol = 6e-5f;
-constexpr float kSnTol = 6e-6f;
-constexpr float kSnCap = 4.f;
-// windows with pixels that are not finite, or too large: as there
-template <bool PLANES>
-__host__ __device__ constexpr float max_energy() { return PLANES ? 3.4e38f : 3e38f / (8.f * (float)N * (float)kThreads); }
-enum { kBadHuge = 1, kBadNan = 2 };
-#define kNegInf64 (-__int_as_float(0x7f800000))
 
 // base-8 digit reversal of a 6-bit index (an involution)
 __device__ __forceinline__ int dr(int v) { return ((v & 7) << 3) | (v >> 3); }
@@ -271,47 +263,6 @@ __device__ __forceinline__ void window_origin(const PivParams& p, int w, int& bx
     }
 }
 
-// a three-source max and a max
-__device__ __forceinline__ float max4(float a, float b, float c, float d)
-{
-    float m;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(fmaxf(c, d)));
-    return m;
-}
-
-// Running top-2 of strict 4-neighbour maxima (find_peaks) plus the largest
-// value whose strict-maximum decision is within dlt of flipping.
-struct Top2 {
-    float t0, t1, umax;
-    int key;
-    __device__ __forceinline__ void init()
-    {
-        t0 = t1 = umax = kNegInf64;
-        key = 0;
-    }
-    __device__ __forceinline__ void add(float c, float m, float dlt, int k)
-    {
-        const float dd = m - c;
-        umax = fabsf(dd) <= dlt ? fmaxf(umax, c) : umax;
-        const float v = dd < 0.f ? c : kNegInf64;
-        t1 = fmaxf(t1, fminf(t0, v));
-        key = v > t0 ? k : key;
-        t0 = fmaxf(t0, v);
-    }
-    // with the lanes o away (ties to the lowest row-major index)
-    __device__ __forceinline__ void merge(int o)
-    {
-        const float o0 = __shfl_xor_sync(0xffffffffu, t0, o);
-        const float o1 = __shfl_xor_sync(0xffffffffu, t1, o);
-        const int ok = __shfl_xor_sync(0xffffffffu, key, o);
-        const bool take = (o0 > t0) || (o0 == t0 && ok < key);
-        t1 = fmaxf(fmaxf(t1, o1), fminf(t0, o0));
-        key = take ? ok : key;
-        t0 = fmaxf(t0, o0);
-        umax = fmaxf(umax, __shfl_xor_sync(0xffffffffu, umax, o));
-    }
-};
-
 extern __shared__ float2 w64_dyn_smem[];
 
 // One task: windows 2 blk and 2 blk + 1 of pair p, run by the whole CTA.
@@ -408,7 +359,7 @@ __device__ __forceinline__ void w64_task(const PivParams& p, const int blk)
             }
             if constexpr (sizeof(PixT) >= 4) {
                 const float e = energy.x + energy.y;
-                if (__syncthreads_or(!(e < max_energy<PLANES>()))) {
+                if (__syncthreads_or(!(e < max_energy<PLANES>(W, kThreads)))) {
                     bad |= (__syncthreads_or(e != e) ? kBadNan : kBadHuge) << (2 * h);
                     energy = before;
                     for (int i = t >> 6; i < W; i += kThreads / W) T[x * LD + i] = make_float2(0.f, 0.f);
@@ -522,8 +473,8 @@ __device__ __forceinline__ void w64_task(const PivParams& p, const int blk)
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-        s[0].merge(o);
-        s[1].merge(o);
+        s[0].merge(s[0].across(o));
+        s[1].merge(s[1].across(o));
     }
     if (lane < 2) s_top[lane][warp] = lane ? s[1] : s[0];
     __syncthreads();
@@ -532,16 +483,15 @@ __device__ __forceinline__ void w64_task(const PivParams& p, const int blk)
     if (warp < 2 && (warp == 0 || valid1)) {
         const int h = warp, w = w0 + h;
         Top2 g = s_top[h][lane & (kWarps - 1)];
-        g.merge(4);
-        g.merge(2);
-        g.merge(1);
+#pragma unroll
+        for (int o = kWarps / 2; o > 0; o >>= 1) g.merge(g.across(o));
         const float ped = s_ped[h];
         auto val = [&](int ys, int xs) -> float {
             const float2 v = cell(ys, xs);
             return h ? v.y : v.x;
         };
         const int bad_h = (bad >> (2 * h)) & 3;
-        const bool has2 = bad_h == 0 && g.t1 > kNegInf64;
+        const bool has2 = bad_h == 0 && g.t1 > kNegInf;
         const int px = has2 ? g.key % W : W / 2, py = has2 ? g.key / W : W / 2;
         const float vc = val(py, px), vl = val(py, px - 1), vr = val(py, px + 1);
         const float vu = val(py - 1, px), vd = val(py + 1, px);
@@ -565,7 +515,7 @@ __device__ __forceinline__ void w64_task(const PivParams& p, const int blk)
             if (bad_h != 0) {
                 certain = bad_h == kBadNan;
             } else if (!has2) {
-                certain = !(g.umax > kNegInf64);
+                certain = !(g.umax > kNegInf);
             } else {
                 const float C = vc + ped, L = vl + ped, R = vr + ped, U = vu + ped, D = vd + ped;
                 const float nan = __int_as_float(0x7fffffff);
