@@ -188,7 +188,7 @@ piv_adjoint_kernel(const PivParams p, const int32_t* __restrict__ peaks, const f
 {
     using L = layout<W>;
     constexpr int m = W - 1;
-    __shared__ float sm[L::WPW > 1 ? 2 * W * L::WPW : 1];
+    __shared__ __align__(8) float sm[L::WPW > 1 ? 2 * W * L::WPW : 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int wib = warp % L::WPW;                       // warp of its window
     const int64_t w = (int64_t)blockIdx.x * (kWarps / L::WPW) + warp / L::WPW;
