@@ -194,11 +194,11 @@ extern "C" int opiv_process_pair_device_noalloc(const void* d_frame_a, const voi
     k.flag_count = reinterpret_cast<unsigned int*>(scratch + kOffCount);
     k.flag_list = reinterpret_cast<int32_t*>(scratch + kOffList);
     k.flag_room = (int32_t)n;
-    // planes of flagged windows: what this grid leaves of the list's room
+    // records of flagged windows: what this grid leaves of the list's room
     const size_t used = ((size_t)n * sizeof(int32_t) + 15) / 16 * 16;
     const size_t left = sizeof(int32_t) * (size_t)kNoAllocMaxWindows - std::min(used, sizeof(int32_t) * (size_t)kNoAllocMaxWindows);
-    k.flag_planes = reinterpret_cast<float*>(scratch + kOffList + used);
-    k.flag_cap = (int32_t)std::min<size_t>((size_t)n, left / (sizeof(float) * flag_record_floats((int)ia)));
+    k.flag_recs = reinterpret_cast<flag_record*>(scratch + kOffList + used);
+    k.flag_cap = (int32_t)std::min<size_t>((size_t)n, left / sizeof(flag_record));
     const double2* tw = reinterpret_cast<const double2*>(scratch + (ia == 16 ? kOffTw16 : kOffTw32));
     k.tw_fwd = tw;
     k.tw_rev = tw + ia;

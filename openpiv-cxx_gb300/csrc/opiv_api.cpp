@@ -114,20 +114,6 @@ std::vector<double2> reference_twiddles(uint32_t n, int dir)
 int exact_blocks(int device) { return 2 * device_sm_count(device); }
 int exact_all_blocks(int device) { return 8 * device_sm_count(device); }
 
-// Flagged windows whose planes a pass keeps for refine_window: one in eight
-// of 16 px windows (REAL mode with the limited search flags up to 13 %, other
-// fields up to 4 %), one in 32 of larger ones (below 1 %), 16 MiB at most; the
-// exact kernel decides those beyond from the frames alone.
-int32_t flag_capacity(int64_t n_win, uint32_t ia)
-{
-    const int64_t room = (int64_t)(16u << 20) / (int64_t)(sizeof(float) * flag_record_floats((int)ia));
-    return (int32_t)std::min({ n_win, 64 + n_win / (ia <= 16 ? 8 : 32), room });
-}
-size_t flag_plane_bytes(int32_t cap, uint32_t ia)
-{
-    return sizeof(float) * flag_record_floats((int)ia) * (size_t)cap;
-}
-
 // Rows of a host frame to the device; one plain copy where they are packed on
 // both sides: a 2-D copy from pageable memory took 56 us more (the multi-pass
 // call over a 2048 x 1536 u16 pair 366 us, 254 with plain copies).
@@ -199,7 +185,7 @@ struct opiv_plan {
     int32_t* d_peak = nullptr;
     unsigned int* d_flag_count = nullptr;
     int32_t* d_flag_list = nullptr;
-    float* d_flag_planes = nullptr;     // planes of the first flag_cap flagged windows
+    flag_record* d_flag_recs = nullptr; // a record for every window (none in tensor-core-only plans)
     int32_t flag_cap = 0;
     double2* d_tw = nullptr;            // forward then reverse, ia entries each
     bool flags = false;                 // the last pass was an FP32 one: d_flag_count[2] is its count
@@ -222,7 +208,7 @@ struct opiv_plan {
     cudaStream_t cs2 = nullptr;                 // compute stream of odd pairs
     unsigned int* p_flag_count[kPipeSlots] = {};
     int32_t* p_flag_list[kPipeSlots] = {};
-    float* p_flag_planes[kPipeSlots] = {};
+    flag_record* p_flag_recs[kPipeSlots] = {};
     void* p_fa[kPipeSlots] = {};
     void* p_fb[kPipeSlots] = {};
     opiv_vector* p_vec[kPipeSlots] = {};
@@ -269,7 +255,7 @@ void plan_free(opiv_plan* p)
     for (int k = 0; k < opiv_plan::kPipeSlots; ++k) {
         cudaFree(p->p_flag_count[k]);
         cudaFree(p->p_flag_list[k]);
-        cudaFree(p->p_flag_planes[k]);
+        cudaFree(p->p_flag_recs[k]);
     }
     if (p->up) cudaStreamDestroy(p->up);
     if (p->down) cudaStreamDestroy(p->down);
@@ -295,7 +281,7 @@ PivParams base_params(const opiv_plan* p)
     k.kappa = kKappa;
     k.flag_count = p->d_flag_count;
     k.flag_list = p->d_flag_list;
-    k.flag_planes = p->d_flag_planes;
+    k.flag_recs = p->d_flag_recs;
     k.flag_cap = p->flag_cap;
     k.flag_room = (int32_t)p->n_win;
     k.tw_fwd = p->d_tw;
@@ -306,7 +292,7 @@ PivParams base_params(const opiv_plan* p)
 // One pass: FP32 kernel over all windows, then the exact pass over the
 // flagged ones.  Two kernel launches.  `prev` (may be null): the previous
 // pass of a multi-pass chain, whose integer displacements offset frame B.
-// flag_count / flag_list / flag_planes: the exact pass's scratch (null: the
+// flag_count / flag_list / flag_recs: the exact pass's scratch (null: the
 // plan's own; passes that may run concurrently need their own).
 // The parameters of one pass of plan p over frames fa, fb; `prev`: the
 // previous pass of a multi-pass chain (window offsetting) or null.
@@ -336,13 +322,13 @@ PivParams pass_params(const opiv_plan* p, const void* fa, const void* fb, size_t
 int run_pass(opiv_plan* p, const void* fa, const void* fb, size_t pitch, opiv_vector* vec,
              int32_t* peak, cudaStream_t s, const opiv_plan* prev = nullptr,
              unsigned int* flag_count = nullptr, int32_t* flag_list = nullptr,
-             float* flag_planes = nullptr)
+             flag_record* flag_recs = nullptr)
 {
     PivParams k = pass_params(p, fa, fb, pitch, vec, peak, prev);
     if (flag_count) {
         k.flag_count = flag_count;
         k.flag_list = flag_list;
-        k.flag_planes = flag_planes;
+        k.flag_recs = flag_recs;
     }
     if (!flag_count) p->flags = p->precision == OPIV_PREC_FP32;
     if (is_tc(p->precision)) {
@@ -516,7 +502,7 @@ int plan_create(opiv_plan** out, uint32_t img_w, uint32_t img_h, int dtype, uint
         return done(cuda_fail(e, "cudaStreamCreate"));
     // one allocation for the plan's outputs and scratch (each costs about as
     // much as all of them together)
-    if (!tc_only) p->flag_cap = flag_capacity(p->n_win, ia);   // the tensor-core path flags nothing
+    if (!tc_only) p->flag_cap = (int32_t)p->n_win;   // the tensor-core path flags nothing
     size_t bytes = 0;
     auto part = [&](size_t size) {
         const size_t at = bytes;
@@ -525,13 +511,13 @@ int plan_create(opiv_plan** out, uint32_t img_w, uint32_t img_h, int dtype, uint
     };
     const size_t at_vec = part(sizeof(opiv_vector) * p->n_win), at_peak = part(sizeof(int32_t) * p->n_win);
     const size_t at_count = part(kFlagCounters * sizeof(unsigned int)), at_list = part(sizeof(int32_t) * p->n_win);
-    const size_t at_planes = part(flag_plane_bytes(p->flag_cap, ia)), at_tw = part(sizeof(double2) * 2 * ia);
+    const size_t at_recs = part(sizeof(flag_record) * p->flag_cap), at_tw = part(sizeof(double2) * 2 * ia);
     if ((e = cudaMalloc(&p->d_scratch, bytes)) != cudaSuccess) return done(cuda_fail(e, "cudaMalloc(plan scratch)"));
     p->d_vec = reinterpret_cast<opiv_vector*>(p->d_scratch + at_vec);
     p->d_peak = reinterpret_cast<int32_t*>(p->d_scratch + at_peak);
     p->d_flag_count = reinterpret_cast<unsigned int*>(p->d_scratch + at_count);
     p->d_flag_list = reinterpret_cast<int32_t*>(p->d_scratch + at_list);
-    p->d_flag_planes = reinterpret_cast<float*>(p->d_scratch + at_planes);
+    p->d_flag_recs = reinterpret_cast<flag_record*>(p->d_scratch + at_recs);
     p->d_tw = reinterpret_cast<double2*>(p->d_scratch + at_tw);
     if ((e = cudaMemsetAsync(p->d_flag_count, 0, kFlagCounters * sizeof(unsigned int), p->stream)) != cudaSuccess)
         return done(cuda_fail(e, "cudaMemset"));
@@ -682,7 +668,7 @@ int opiv_process_pairs(opiv_plan* plan, int64_t n_pairs, const void* const* fram
                 break;
             if ((e = cudaMalloc(&plan->p_flag_list[k], sizeof(int32_t) * plan->n_win)) != cudaSuccess) break;
             if (plan->flag_cap > 0)
-                e = cudaMalloc(&plan->p_flag_planes[k], flag_plane_bytes(plan->flag_cap, plan->ia));
+                e = cudaMalloc(&plan->p_flag_recs[k], sizeof(flag_record) * plan->flag_cap);
         }
         if (e == cudaSuccess) e = cudaStreamSynchronize(plan->stream);   // both compute streams rely on the counters
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&plan->up, cudaStreamNonBlocking);
@@ -718,7 +704,7 @@ int opiv_process_pairs(opiv_plan* plan, int64_t n_pairs, const void* const* fram
         if (i >= S) CUDA_TRY(cudaStreamWaitEvent(cs, plan->ev_down[k], 0));
         const int rc = run_pass(plan, plan->p_fa[k], plan->p_fb[k], row, plan->p_vec[k],
                                 out_peak ? plan->p_peak[k] : nullptr, cs, nullptr,
-                                plan->p_flag_count[k], plan->p_flag_list[k], plan->p_flag_planes[k]);
+                                plan->p_flag_count[k], plan->p_flag_list[k], plan->p_flag_recs[k]);
         if (rc != OPIV_OK) return done(rc);
         CUDA_TRY(cudaEventRecord(plan->ev_done[k], cs));
         CUDA_TRY(cudaStreamWaitEvent(plan->down, plan->ev_done[k], 0));
@@ -902,7 +888,7 @@ struct batch_queue_pass {
     std::vector<PivQueue> groups;       // host copies, passed by value at launch
     unsigned int* d_ctr = nullptr;      // per group: dequeue head, flagged windows
     int32_t* d_flags = nullptr;         // per group: its flag list (combined window numbers)
-    float* d_planes = nullptr;          // per group: planes of its first flagged windows
+    flag_record* d_recs = nullptr;      // per group: its flagged windows' records
     PivParams* d_items = nullptr;       // per group: its descriptors (kQueueMaxItems slots)
     uint8_t* d_task_item = nullptr;     // per group: the pair of every task
     int ia = 0, dtype = 0, mode = 0, limit = 0;
@@ -957,7 +943,7 @@ void batch_free_queue(opiv_batch* b)
     for (batch_queue_pass& q : b->qp) {
         cudaFree(q.d_ctr);
         cudaFree(q.d_flags);
-        cudaFree(q.d_planes);
+        cudaFree(q.d_recs);
         cudaFree(q.d_items);
         cudaFree(q.d_task_item);
     }
@@ -1010,8 +996,7 @@ int batch_queue_setup(opiv_batch* b)
             break;
         }
         q.groups.resize(n_groups);
-        std::vector<int64_t> flag_off(n_groups + 1, 0);   // each group's flag list in d_flags
-        std::vector<int64_t> plane_off(n_groups + 1, 0);  // each group's records in d_planes
+        std::vector<int64_t> flag_off(n_groups + 1, 0);   // each group's place in d_flags and d_recs
         std::vector<int64_t> task_off(n_groups + 1, 0);   // each group's task pairs in d_task_item
         std::vector<uint8_t> task_item;
         const size_t px = px_bytes(q.dtype);
@@ -1045,15 +1030,13 @@ int batch_queue_setup(opiv_batch* b)
             pq.first_task[pq.n_items] = (int)tasks;
             pq.first_win[pq.n_items] = (int)wins;
             flag_off[g + 1] = flag_off[g] + (wins > 0 ? wins : 1);
-            plane_off[g + 1] = plane_off[g] + flag_capacity(wins, q.ia);
             task_off[g + 1] = task_off[g] + tasks;
         }
         if (rc != OPIV_OK) break;
         cudaError_t e;
         if ((e = cudaMalloc(&q.d_ctr, 2 * sizeof(unsigned int) * n_groups)) != cudaSuccess ||
             (e = cudaMalloc(&q.d_flags, sizeof(int32_t) * flag_off[n_groups])) != cudaSuccess ||
-            (e = cudaMalloc(&q.d_planes, flag_plane_bytes((int32_t)std::max<int64_t>(1, plane_off[n_groups]), q.ia))) !=
-                cudaSuccess ||
+            (e = cudaMalloc(&q.d_recs, sizeof(flag_record) * flag_off[n_groups])) != cudaSuccess ||
             (e = cudaMalloc(&q.d_items, sizeof(PivParams) * kQueueMaxItems * n_groups)) != cudaSuccess ||
             (e = cudaMalloc(&q.d_task_item, task_item.size() + 1)) != cudaSuccess) {
             rc = cuda_fail(e, "cudaMalloc(work queue)");
@@ -1067,9 +1050,8 @@ int batch_queue_setup(opiv_batch* b)
             for (int j = 0; j < pq.n_items; ++j) {   // the group's one flag list
                 pq.items[j].flag_count = q.d_ctr + 2 * g + 1;
                 pq.items[j].flag_list = q.d_flags + flag_off[g];
-                pq.items[j].flag_planes = q.d_planes + plane_off[g] * flag_record_floats(q.ia);
-                pq.items[j].flag_cap = (int32_t)(plane_off[g + 1] - plane_off[g]);
-                pq.items[j].flag_room = (int32_t)(flag_off[g + 1] - flag_off[g]);
+                pq.items[j].flag_recs = q.d_recs + flag_off[g];
+                pq.items[j].flag_cap = pq.items[j].flag_room = (int32_t)(flag_off[g + 1] - flag_off[g]);
             }
             pq.items_g = q.d_items + (size_t)kQueueMaxItems * g;
             pq.task_item = q.d_task_item + task_off[g];
@@ -1091,8 +1073,9 @@ int batch_queue_setup(opiv_batch* b)
             break;
         }
         if (q.max_ctas < 1) q.max_ctas = 1;
-        // flagged windows are few but each costs ~0.1 ms of FP64 latency in one
-        // CTA; as many run at once as fit, so the pass waits about one round
+        // flagged windows are few, but each is one CTA's chain: some 10 us of
+        // exact sums, 40 us (16 px) to 0.3 ms (64 px) where it takes the FP64
+        // transforms; as many run at once as fit, so the pass waits about one round
         q.exact_blocks = exact_queue_max_ctas_per_sm(q.ia) * b->sms;
         q.ctas_per_sm = b->tune_ctas[k];
         q.chunk = b->tune_chunk[k];

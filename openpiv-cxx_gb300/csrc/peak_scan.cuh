@@ -4,6 +4,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "piv_kernels.h"
+
 namespace opiv {
 
 // A window is decided by an FP32 kernel only if the error bound of its
@@ -84,5 +86,86 @@ struct Top2 {
         return r;
     }
 };
+
+// The record of a flagged window, by LANES lanes of a warp; every lane calls
+// it, with its group's arguments (rec null: nothing is written).  tile: both
+// planes before the quadrant swap, the window's in component h; lines W + 1
+// apart, of rows, or of columns where COLS.  dlt: the bound, zero for none.
+// Scanned: swapped rows SY0 .. SY1 - 1 and columns SX0 .. SX1 - 1.  The order of
+// the cells follows the scan, whichever lane finds them.
+template <int W, int LANES, bool COLS, int SY0, int SY1, int SX0, int SX1>
+__device__ __forceinline__ void record_candidates(const float2* tile, int h, float dlt, flag_record* rec)
+{
+    constexpr int NX = SX1 - SX0, NC = (SY1 - SY0) * NX;
+    const int lane = (int)threadIdx.x & 31, gl = lane % LANES;
+    auto cell = [&](int y, int x) -> float {
+        y = (y + W / 2) & (W - 1);
+        x = (x + W / 2) & (W - 1);
+        const float2 v = tile[COLS ? x * (W + 1) + y : y * (W + 1) + x];
+        return h ? v.y : v.x;
+    };
+    auto rise = [&](int y, int x, float c) {   // highest neighbour minus the cell
+        return max4(cell(y - 1, x), cell(y + 1, x), cell(y, x - 1), cell(y, x + 1)) - c;
+    };
+    // the two highest cells that are maxima whatever the rounding: nothing
+    // below the second of them (less the bound) matters
+    float s0 = kNegInf, s1 = kNegInf;
+#pragma unroll(LANES == 32 ? 4 : 2)
+    for (int b = 0; b < NC; b += LANES) {
+        const int i = b + gl, y = SY0 + i / NX, x = SX0 + i % NX;   // past the last: other cells of the tile
+        const float c = cell(y, x);
+        const float v = i < NC && rise(y, x, c) < -dlt ? c : kNegInf;
+        s1 = fmaxf(s1, fminf(s0, v));
+        s0 = fmaxf(s0, v);
+    }
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) {
+        const float q0 = __shfl_xor_sync(0xffffffffu, s0, o), q1 = __shfl_xor_sync(0xffffffffu, s1, o);
+        s1 = fmaxf(fmaxf(s1, q1), fminf(s0, q0));
+        s0 = fmaxf(s0, q0);
+    }
+    const float floor_c = s1 - dlt;
+    int n = 0;
+#pragma unroll(LANES == 32 ? 4 : 2)
+    for (int b = 0; b < NC; b += LANES) {
+        const int i = b + gl, y = SY0 + i / NX, x = SX0 + i % NX;
+        const float c = cell(y, x);
+        const bool high = i < NC && c >= floor_c;
+        if (!__any_sync(0xffffffffu, high)) continue;
+        const bool mine = high && rise(y, x, c) <= dlt;
+        const unsigned group = __ballot_sync(0xffffffffu, mine) >> (lane - gl) & (0xffffffffu >> (32 - LANES));
+        const int at = n + __popc(group & ((1u << gl) - 1u));
+        if (mine && rec != nullptr && at < kMaxCand) rec->key[at] = (uint16_t)(y * W + x);
+        n += __popc(group);
+    }
+    if (rec != nullptr && gl == 0) {
+        rec->n = n;
+        rec->dlt = dlt;
+    }
+}
+
+// Few windows are flagged, so the records are functions of their own: the
+// others' code stays small (4096 x 4096, 32 px at step 8: 707 us, 716 inlined).
+// record_group: a window by LANES lanes (32 px: a warp has two windows, and the
+// loop of record_warp costs the kernel 8 us there).  record_warp: one window after
+// the other by the whole warp; a lane whose slot is not negative speaks for a
+// window (16 px, 2048 x 1536 at step 8: 42.5 us; 45.7 by a window's own eight lanes,
+// whose scan the pass waits for).
+template <int W, int LANES, bool COLS, int SY0, int SY1, int SX0, int SX1>
+__device__ __noinline__ void record_group(const float2* tile, int h, float dlt, flag_record* rec)
+{
+    record_candidates<W, LANES, COLS, SY0, SY1, SX0, SX1>(tile, h, dlt, rec);
+}
+template <int W, bool COLS, int SY0, int SY1, int SX0, int SX1>
+__device__ __noinline__ void record_warp(const float2* tile, int h, float dlt, int slot, flag_record* recs)
+{
+    for (unsigned todo = __ballot_sync(0xffffffffu, slot >= 0); todo != 0; todo &= todo - 1) {
+        const int from = __ffs((int)todo) - 1;
+        record_candidates<W, 32, COLS, SY0, SY1, SX0, SX1>(
+            reinterpret_cast<const float2*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(tile), from)),
+            __shfl_sync(0xffffffffu, h, from), __shfl_sync(0xffffffffu, dlt, from),
+            recs + __shfl_sync(0xffffffffu, slot, from));
+    }
+}
 
 }  // namespace opiv

@@ -282,10 +282,10 @@ __device__ __forceinline__ void exact_window(const PivParams& p, const int64_t w
 // sums, sum_p a[p] b[p + lag]: whole numbers for 8/16-bit frames (at most
 // 2^44, kept in 64 bits), FP64 sums for float frames.  So instead of three
 // 2-D transforms in FP64 (about 160,000 FP64 operations for a 32 px window at
-// two per cycle and SM: 40 us for one CTA at best), the CTA takes the FP32
-// plane that the window was flagged with, finds every cell that could be one
-// of the two highest maxima within the FP32 error bound, and evaluates those
-// cells and their neighbours exactly.  In units of W^2 times a plane value,
+// two per cycle and SM: 40 us for one CTA at best), the CTA takes the cells
+// of the FP32 plane that could be one of the two highest maxima within its
+// error bound (the window's record), and evaluates those cells and their
+// neighbours exactly.  In units of W^2 times a plane value,
 // REAL mode's plane (spectrum column 0 and rows 0, W/2 left out) is
 //   V = W^2 R - W (rows + columns + (-1)^dy alternating)
 //         + Sa Sb + (-1)^dy Ta Tb,
@@ -300,13 +300,9 @@ __device__ __forceinline__ void exact_window(const PivParams& p, const int64_t w
 // at step 8 (78 flagged) 48 -> 9 us; 2048 x 2048, 64 px at step 16 (2 flagged)
 // 360 -> 20 us; none flagged 3 us.  What is left is a chain of dependent loads,
 // block barriers and FP64 logarithms of one window.
-constexpr int kMaxCand = 16;
-
 struct refine_shared {
     long long val[5 * kMaxCand];   // or doubles: centre, left, right, up, down
-    float top0[kThreads / 32], top1[kThreads / 32];
     int key[kMaxCand];
-    int count;
     int ok;
 };
 
@@ -319,21 +315,20 @@ __device__ __forceinline__ T warp_total(T v)
 
 template <typename PixT>
 __device__ __forceinline__ bool refine_window(const PivParams& p, const int64_t w, const int W, const int mode,
-                                              const int sy0, const int sy1, const int sx0, const int sx1,
-                                              const float* rec, unsigned char* smem, refine_shared& rs)
+                                              const flag_record& rec, unsigned char* smem, refine_shared& rs)
 {
     constexpr bool kFloat = sizeof(PixT) == 4;
     using Px = typename std::conditional<kFloat, double, uint32_t>::type;
     using Acc = typename std::conditional<kFloat, double, long long>::type;
     const int t = threadIdx.x, T = blockDim.x, lane = t & 31, warp = t >> 5, warps = T >> 5;
     const int N = W * W, m = W - 1, lg = 31 - __clz(W);
-    const float dlt = rec[N];
-    if (!(dlt > 1e-30f && dlt < 1e30f)) return false;   // block-uniform; also blank windows and NaN
+    const float dlt = rec.dlt;
+    const int n = rec.n;
+    if (!(dlt > 1e-30f && dlt < 1e30f) || n > kMaxCand) return false;   // block-uniform
 
     Px* A = reinterpret_cast<Px*>(smem);
     Px* B = A + N;
-    float* C = reinterpret_cast<float*>(B + N);
-    Acc* prof = reinterpret_cast<Acc*>(C + N);   // REAL: 6 W sums
+    Acc* prof = reinterpret_cast<Acc*>(B + N);   // REAL: 6 W sums
     int bx, by, ox, oy;
     window_origin(p, w, bx, by);
     b_offset(p, W, bx, by, ox, oy);
@@ -345,38 +340,10 @@ __device__ __forceinline__ bool refine_window(const PivParams& p, const int64_t 
             const int y = i >> lg, x = i & m;
             A[i] = (Px)__ldg(fa + (size_t)(by + y) * pitch + bx + x);
             B[i] = (Px)__ldg(fb + (size_t)(by + oy + y) * pitch + bx + ox + x);
-            C[i] = rec[i];
         }
     }
-    if (t == 0) rs.count = 0;
+    if (t < kMaxCand) rs.key[t] = rec.key[t] & (N - 1);
     __syncthreads();
-
-    // the two highest cells that are maxima whatever the rounding: nothing
-    // below the second of them (less the bound) matters
-    const float ninf = -__int_as_float(0x7f800000);
-    auto scanned = [&](int k) {
-        const int y = k >> lg, x = k & m;
-        return y >= sy0 && y < sy1 && x >= sx0 && x < sx1;
-    };
-    auto rise = [&](int k) {   // highest neighbour minus the cell
-        return fmaxf(fmaxf(C[k - 1], C[k + 1]), fmaxf(C[k - W], C[k + W])) - C[k];
-    };
-    float s0 = ninf, s1 = ninf;
-    for (int k = t; k < N; k += T) {
-        if (!scanned(k)) continue;
-        const float c = rise(k) < -dlt ? C[k] : ninf;
-        s1 = fmaxf(s1, fminf(s0, c));
-        s0 = fmaxf(s0, c);
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        const float q0 = __shfl_xor_sync(0xffffffffu, s0, o), q1 = __shfl_xor_sync(0xffffffffu, s1, o);
-        s1 = fmaxf(fmaxf(s1, q1), fminf(s0, q0));
-        s0 = fmaxf(s0, q0);
-    }
-    if (lane == 0) {
-        rs.top0[warp] = s0;
-        rs.top1[warp] = s1;
-    }
     if (mode == kModeReal) {
         // row sums of a and b, column sums, (-1)^y-weighted column sums
         for (int i = t; i < 4 * W; i += T) {
@@ -396,25 +363,7 @@ __device__ __forceinline__ bool refine_window(const PivParams& p, const int64_t 
                 prof[(4 + (i & 1)) * W + l] = h;
             }
         }
-    }
-    __syncthreads();
-    float g0 = ninf, g1 = ninf;
-    for (int i = 0; i < warps; ++i) {
-        g1 = fmaxf(fmaxf(g1, rs.top1[i]), fminf(g0, rs.top0[i]));
-        g0 = fmaxf(g0, rs.top0[i]);
-    }
-    const float floor_c = g1 - dlt;
-    for (int k = t; k < N; k += T) {
-        if (scanned(k) && C[k] >= floor_c && rise(k) <= dlt) {
-            const int n = atomicAdd(&rs.count, 1);
-            if (n < kMaxCand) rs.key[n] = k;
-        }
-    }
-    __syncthreads();
-    const int n = rs.count;
-    if (n > kMaxCand) {
-        __syncthreads();   // the next window resets the count
-        return false;
+        __syncthreads();
     }
 
     // exact values, one warp per value
@@ -549,7 +498,8 @@ __device__ __forceinline__ void scan_range(int W, int limit, int& sy0, int& sy1,
 }
 
 // LIST: the windows of flag_list (the pass after the FP32 kernel), exact
-// sums first; otherwise every window in FP64.
+// sums first, for all of them or none (the list's order is the order of
+// arrival, so the first flag_cap of more would be other windows each time); otherwise every window in FP64.
 template <typename PixT, bool LIST>
 __global__ void __launch_bounds__(kThreads)
 piv_exact_kernel(const PivParams p, int W, int mode, int limit)
@@ -566,10 +516,8 @@ piv_exact_kernel(const PivParams p, int W, int mode, int limit)
         const int64_t w = LIST ? (int64_t)p.flag_list[item] : item;
         if constexpr (LIST) {
             __shared__ refine_shared rs;
-            if (item < p.flag_cap &&
-                refine_window<PixT>(p, w, W, mode, sy0, sy1, sx0, sx1,
-                                    p.flag_planes + (size_t)item * flag_record_floats(W),
-                                    reinterpret_cast<unsigned char*>(sm), rs)) {
+            if (nwork <= p.flag_cap &&
+                refine_window<PixT>(p, w, W, mode, p.flag_recs[item], reinterpret_cast<unsigned char*>(sm), rs)) {
                 ++settled;
                 continue;
             }
@@ -587,7 +535,7 @@ piv_exact_kernel(const PivParams p, int W, int mode, int limit)
         }
         if (threadIdx.x == 0 && atomicAdd(p.flag_count + 1, 1u) == gridDim.x - 1) {
             p.flag_count[2] = (unsigned int)nwork;
-            p.flag_count[4] = atomicExch(p.flag_count + 3, 0u);
+            p.flag_count[4] = nwork > 0 ? atomicExch(p.flag_count + 3, 0u) : 0u;   // (a round trip to memory)
             p.flag_count[1] = 0u;
             p.flag_count[0] = 0u;
         }
@@ -617,10 +565,8 @@ piv_exact_queue_kernel(const __grid_constant__ PivQueue q, int W, int mode, int 
         }
         const PivParams& p = q.items[lo];
         const int64_t w = (int64_t)(g - q.first_win[lo]);
-        if (item < p.flag_cap &&
-            refine_window<PixT>(p, w, W, mode, sy0, sy1, sx0, sx1,
-                                p.flag_planes + (size_t)item * flag_record_floats(W),
-                                reinterpret_cast<unsigned char*>(sm), rs))
+        if (nwork <= p.flag_cap &&
+            refine_window<PixT>(p, w, W, mode, p.flag_recs[item], reinterpret_cast<unsigned char*>(sm), rs))
             continue;
         exact_window<PixT>(p, w, W, mode, sy0, sy1, sx0, sx1, sm, sm + W * W, row_count, &total_cand);
     }

@@ -633,13 +633,15 @@ __device__ __forceinline__ void fp32_task(const PivParams& p, const int task, fl
             if (at < (unsigned int)p.flag_cap) slot = (int)at;
         }
     }
-    // a flagged window hands its plane on
-    if (!PLANES) slot = __shfl_sync(0xffffffffu, slot, 0, HL);
-    if (!PLANES && slot >= 0) {
-        float* rec = p.flag_planes + (size_t)slot * flag_record_floats(W);
-#pragma unroll 1
-        for (int i = hl; i < N; i += HL) rec[i] = cell(i / W + W / 2, i % W + W / 2);
-        if (hl == 0) rec[N] = bad_h == 0 ? dlt : 0.f;   // without a bound: to the FP64 transforms
+    // a flagged window hands its candidates on
+    if (!PLANES && __any_sync(0xffffffffu, slot >= 0)) {
+        const float bound = bad_h == 0 ? dlt : 0.f;   // without one: to the FP64 transforms
+        if constexpr (W == 16) {
+            record_warp<W, false, SY0, SY1, SX0, SX1>(S, h, bound, slot, p.flag_recs);
+        } else {
+            slot = __shfl_sync(0xffffffffu, slot, 0, HL);
+            record_group<W, HL, false, SY0, SY1, SX0, SX1>(S, h, bound, slot >= 0 ? p.flag_recs + slot : nullptr);
+        }
     }
 }
 

@@ -552,13 +552,10 @@ __device__ __forceinline__ void w64_task(const PivParams& p, const int blk)
                 if (at < (unsigned int)p.flag_cap) slot = (int)at;
             }
         }
-        // a flagged window hands its plane on
+        // a flagged window hands its candidates on
         if (!PLANES) slot = __shfl_sync(0xffffffffu, slot, 0);
-        if (!PLANES && slot >= 0) {
-            float* rec = p.flag_planes + (size_t)slot * flag_record_floats(W);
-            for (int i = lane; i < N; i += 32) rec[i] = val(i >> 6, i & 63);
-            if (lane == 0) rec[N] = bad_h == 0 ? dlt : 0.f;   // without a bound: to the FP64 transforms
-        }
+        if (!PLANES && slot >= 0)   // without a bound: to the FP64 transforms
+            record_group<W, 32, true, SY0, SY1, SX0, SX1>(T, h, bad_h == 0 ? dlt : 0.f, p.flag_recs + slot);
     }
 }
 

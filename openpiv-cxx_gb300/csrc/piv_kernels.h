@@ -10,6 +10,20 @@ namespace opiv {
 enum { kModeReal = OPIV_CORR_REAL, kModeComplex = OPIV_CORR_COMPLEX };
 enum { kU8 = OPIV_U8, kU16 = OPIV_U16, kF32 = OPIV_F32, kF64 = 3 /* internal: batch API */ };
 
+// What a flagged window hands to the second launch (peak_scan.cuh writes it,
+// refine_window in piv_exact.cu reads it): the error bound of its FP32 plane and
+// the n cells py * W + px that may be one of its two highest maxima within the
+// bound.  The cells and not the plane, so that a pass has room for every window:
+// with planes it did not, and which windows beyond the room went to the FP64
+// transforms was the order of arrival.  n > kMaxCand (no cell kept) or a bound
+// of zero: for the FP64 transforms.
+constexpr int kMaxCand = 16;
+struct flag_record {
+    float dlt;
+    int32_t n;
+    uint16_t key[kMaxCand];
+};
+
 // Everything one pass over an image pair needs on the device.
 struct alignas(16) PivParams {
     const void* fa = nullptr;          // frame A (device), img_h rows of `pitch` bytes
@@ -33,12 +47,12 @@ struct alignas(16) PivParams {
     unsigned int* flag_count = nullptr;
     int32_t* flag_list = nullptr;
     int32_t flag_base = 0;             // added to a flagged window's index (a queue's list)
-    // planes of the first flag_cap flagged windows, by their place in the
-    // list: flag_record_floats(W) floats each, the quadrant-swapped FP32
-    // plane and then its error bound (refine_window in piv_exact.cu)
+    // the flagged windows' records, by their place in the list.  A pass that
+    // flags more windows than flag_cap takes the FP64 transforms for all of
+    // them (the allocation-free call on large grids; plans have one a window).
     int32_t flag_cap = 0;
     int32_t flag_room = 0;             // entries of flag_list
-    float* flag_planes = nullptr;
+    flag_record* flag_recs = nullptr;
     float kappa = 16.f;                // FP32 error-bound factor
     // debug / per-window API outputs
     float* planes = nullptr;           // FP32 kernel: n_win * W * W (mean-free part)
@@ -91,10 +105,6 @@ inline cudaError_t launch_dependent(void (*kernel)(P...), unsigned int blocks, i
 #ifdef __CUDACC__
 __device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 #endif
-
-// Floats of a flagged window's record: the plane, its error bound, padding
-// to 16 bytes.
-__host__ __device__ constexpr int flag_record_floats(int w) { return w * w + 4; }
 
 // Tensor-core DFT-GEMM kernels (piv_tc.cu): 16, 32, 48 and 64 px windows
 // (32: piv_tc_kernel.cuh; the others: piv_tcg_kernel.cuh), u8/u16 frames,
