@@ -114,6 +114,10 @@ std::vector<double2> reference_twiddles(uint32_t n, int dir)
 int exact_blocks(int device) { return 2 * device_sm_count(device); }
 int exact_all_blocks(int device) { return 8 * device_sm_count(device); }
 
+// A frame of the library's own: whole 16-byte blocks, so that rows can be read
+// as the blocks that cover them.
+cudaError_t alloc_frame(void** frame, size_t bytes) { return cudaMalloc(frame, (bytes + 15) / 16 * 16); }
+
 // Rows of a host frame to the device; one plain copy where they are packed on
 // both sides: a 2-D copy from pageable memory took 56 us more (the multi-pass
 // call over a 2048 x 1536 u16 pair 366 us, 254 with plain copies).
@@ -294,15 +298,17 @@ PivParams base_params(const opiv_plan* p)
 // pass of a multi-pass chain, whose integer displacements offset frame B.
 // flag_count / flag_list / flag_recs: the exact pass's scratch (null: the
 // plan's own; passes that may run concurrently need their own).
-// The parameters of one pass of plan p over frames fa, fb; `prev`: the
-// previous pass of a multi-pass chain (window offsetting) or null.
-PivParams pass_params(const opiv_plan* p, const void* fa, const void* fb, size_t pitch,
+// The parameters of one pass of plan p over frames fa, fb (`padded`: from
+// alloc_frame); `prev`: the previous pass of a multi-pass chain (window
+// offsetting) or null.
+PivParams pass_params(const opiv_plan* p, const void* fa, const void* fb, size_t pitch, bool padded,
                       opiv_vector* vec, int32_t* peak, const opiv_plan* prev)
 {
     PivParams k = base_params(p);
     k.fa = fa;
     k.fb = fb;
     k.pitch = pitch;
+    k.frames_padded = padded;
     k.out_vec = vec;
     k.out_peak = peak;
     k.out_disp = p->d_disp;
@@ -319,12 +325,12 @@ PivParams pass_params(const opiv_plan* p, const void* fa, const void* fb, size_t
     return k;
 }
 
-int run_pass(opiv_plan* p, const void* fa, const void* fb, size_t pitch, opiv_vector* vec,
+int run_pass(opiv_plan* p, const void* fa, const void* fb, size_t pitch, bool padded, opiv_vector* vec,
              int32_t* peak, cudaStream_t s, const opiv_plan* prev = nullptr,
              unsigned int* flag_count = nullptr, int32_t* flag_list = nullptr,
              flag_record* flag_recs = nullptr)
 {
-    PivParams k = pass_params(p, fa, fb, pitch, vec, peak, prev);
+    PivParams k = pass_params(p, fa, fb, pitch, padded, vec, peak, prev);
     if (flag_count) {
         k.flag_count = flag_count;
         k.flag_list = flag_list;
@@ -591,7 +597,7 @@ int opiv_process_pair_device(opiv_plan* plan, const void* d_fa, const void* d_fb
     int prev = 0;
     cudaGetDevice(&prev);
     cudaSetDevice(plan->device);
-    const int rc = run_pass(plan, d_fa, d_fb, pitch_bytes, d_out_vec, d_out_peak,
+    const int rc = run_pass(plan, d_fa, d_fb, pitch_bytes, false, d_out_vec, d_out_peak,
                             (cudaStream_t)stream);
     cudaSetDevice(prev);
     return rc;
@@ -609,9 +615,9 @@ int opiv_process_pair(opiv_plan* plan, const void* frame_a, const void* frame_b,
     auto done = [&](int s) { cudaSetDevice(prev); return s; };
     cudaError_t e;
     if (!plan->d_fa) {
-        if ((e = cudaMalloc(&plan->d_fa, row * plan->img_h)) != cudaSuccess)
+        if ((e = alloc_frame(&plan->d_fa, row * plan->img_h)) != cudaSuccess)
             return done(cuda_fail(e, "cudaMalloc(frame)"));
-        if ((e = cudaMalloc(&plan->d_fb, row * plan->img_h)) != cudaSuccess)
+        if ((e = alloc_frame(&plan->d_fb, row * plan->img_h)) != cudaSuccess)
             return done(cuda_fail(e, "cudaMalloc(frame)"));
         plan->d_pitch = row;
     }
@@ -620,7 +626,7 @@ int opiv_process_pair(opiv_plan* plan, const void* frame_a, const void* frame_b,
         return done(cuda_fail(e, "upload_frame(frame a)"));
     if ((e = upload_frame(plan->d_fb, plan->d_pitch, frame_b, pitch_bytes, row, plan->img_h, s)) != cudaSuccess)
         return done(cuda_fail(e, "upload_frame(frame b)"));
-    int rc = run_pass(plan, plan->d_fa, plan->d_fb, plan->d_pitch, plan->d_vec,
+    int rc = run_pass(plan, plan->d_fa, plan->d_fb, plan->d_pitch, true, plan->d_vec,
                       out_peak ? plan->d_peak : nullptr, s);
     if (rc != OPIV_OK) return done(rc);
     if ((e = cudaMemcpyAsync(out_vec, plan->d_vec, sizeof(opiv_vector) * plan->n_win,
@@ -655,8 +661,8 @@ int opiv_process_pairs(opiv_plan* plan, int64_t n_pairs, const void* const* fram
     cudaError_t e = cudaSuccess;
     if (!plan->pipe) {
         for (int k = 0; k < opiv_plan::kPipeSlots && e == cudaSuccess; ++k) {
-            if ((e = cudaMalloc(&plan->p_fa[k], row * plan->img_h)) != cudaSuccess) break;
-            if ((e = cudaMalloc(&plan->p_fb[k], row * plan->img_h)) != cudaSuccess) break;
+            if ((e = alloc_frame(&plan->p_fa[k], row * plan->img_h)) != cudaSuccess) break;
+            if ((e = alloc_frame(&plan->p_fb[k], row * plan->img_h)) != cudaSuccess) break;
             if ((e = cudaMalloc(&plan->p_vec[k], sizeof(opiv_vector) * plan->n_win)) != cudaSuccess) break;
             if ((e = cudaMalloc(&plan->p_peak[k], sizeof(int32_t) * plan->n_win)) != cudaSuccess) break;
             if ((e = cudaEventCreateWithFlags(&plan->ev_up[k], cudaEventDisableTiming)) != cudaSuccess) break;
@@ -702,7 +708,7 @@ int opiv_process_pairs(opiv_plan* plan, int64_t n_pairs, const void* const* fram
         CUDA_TRY(cudaEventRecord(plan->ev_up[k], plan->up));
         CUDA_TRY(cudaStreamWaitEvent(cs, plan->ev_up[k], 0));
         if (i >= S) CUDA_TRY(cudaStreamWaitEvent(cs, plan->ev_down[k], 0));
-        const int rc = run_pass(plan, plan->p_fa[k], plan->p_fb[k], row, plan->p_vec[k],
+        const int rc = run_pass(plan, plan->p_fa[k], plan->p_fb[k], row, true, plan->p_vec[k],
                                 out_peak ? plan->p_peak[k] : nullptr, cs, nullptr,
                                 plan->p_flag_count[k], plan->p_flag_list[k], plan->p_flag_recs[k]);
         if (rc != OPIV_OK) return done(rc);
@@ -808,10 +814,11 @@ int opiv_multipass_grid(const opiv_multipass* mp, int pass, int32_t* out_xy, int
     return opiv_plan_grid(mp->passes[pass], out_xy, cap);
 }
 
-int opiv_multipass_process_device(opiv_multipass* mp, const void* d_fa, const void* d_fb,
-                                  size_t pitch_bytes, void* stream)
+namespace {
+
+int multipass_device(opiv_multipass* mp, const void* d_fa, const void* d_fb, size_t pitch_bytes, bool padded,
+                     cudaStream_t s)
 {
-    if (!mp || !d_fa || !d_fb) return fail(OPIV_ERR_ARG, "null argument");
     opiv_plan* first = mp->passes[0];
     if (pitch_bytes < (size_t)first->img_w * px_bytes(first->dtype))
         return fail(OPIV_ERR_ARG, "pitch %zu smaller than a row", pitch_bytes);
@@ -821,11 +828,19 @@ int opiv_multipass_process_device(opiv_multipass* mp, const void* d_fa, const vo
     int rc = OPIV_OK;
     for (size_t k = 0; k < mp->passes.size() && rc == OPIV_OK; ++k) {
         opiv_plan* p = mp->passes[k];
-        rc = run_pass(p, d_fa, d_fb, pitch_bytes, p->d_vec, p->d_peak, (cudaStream_t)stream,
-                      k ? mp->passes[k - 1] : nullptr);
+        rc = run_pass(p, d_fa, d_fb, pitch_bytes, padded, p->d_vec, p->d_peak, s, k ? mp->passes[k - 1] : nullptr);
     }
     cudaSetDevice(prev);
     return rc;
+}
+
+}  // namespace
+
+int opiv_multipass_process_device(opiv_multipass* mp, const void* d_fa, const void* d_fb,
+                                  size_t pitch_bytes, void* stream)
+{
+    if (!mp || !d_fa || !d_fb) return fail(OPIV_ERR_ARG, "null argument");
+    return multipass_device(mp, d_fa, d_fb, pitch_bytes, false, (cudaStream_t)stream);
 }
 
 int opiv_multipass_process(opiv_multipass* mp, const void* frame_a, const void* frame_b,
@@ -842,8 +857,8 @@ int opiv_multipass_process(opiv_multipass* mp, const void* frame_a, const void* 
     auto done = [&](int st) { cudaSetDevice(prev); return st; };
     cudaError_t e;
     if (!mp->d_fa) {
-        if ((e = cudaMalloc(&mp->d_fa, row * first->img_h)) != cudaSuccess) return done(cuda_fail(e, "cudaMalloc(frame)"));
-        if ((e = cudaMalloc(&mp->d_fb, row * first->img_h)) != cudaSuccess) return done(cuda_fail(e, "cudaMalloc(frame)"));
+        if ((e = alloc_frame(&mp->d_fa, row * first->img_h)) != cudaSuccess) return done(cuda_fail(e, "cudaMalloc(frame)"));
+        if ((e = alloc_frame(&mp->d_fb, row * first->img_h)) != cudaSuccess) return done(cuda_fail(e, "cudaMalloc(frame)"));
         mp->d_pitch = row;
     }
     cudaStream_t s = first->stream;
@@ -851,7 +866,7 @@ int opiv_multipass_process(opiv_multipass* mp, const void* frame_a, const void* 
         return done(cuda_fail(e, "upload_frame(frame a)"));
     if ((e = upload_frame(mp->d_fb, mp->d_pitch, frame_b, pitch_bytes, row, first->img_h, s)) != cudaSuccess)
         return done(cuda_fail(e, "upload_frame(frame b)"));
-    const int rc = opiv_multipass_process_device(mp, mp->d_fa, mp->d_fb, mp->d_pitch, s);
+    const int rc = multipass_device(mp, mp->d_fa, mp->d_fb, mp->d_pitch, true, s);
     if (rc != OPIV_OK) return done(rc);
     if ((e = cudaStreamSynchronize(s)) != cudaSuccess) return done(cuda_fail(e, "cudaStreamSynchronize"));
     cudaSetDevice(prev);
@@ -1008,7 +1023,8 @@ int batch_queue_setup(opiv_batch* b)
                 const int i = group_pairs[g][j];
                 const opiv_plan* p = b->pairs[i]->passes[k];
                 const opiv_plan* prev = k ? b->pairs[i]->passes[k - 1] : nullptr;
-                PivParams it = pass_params(p, b->d_fa[i], b->d_fb[i], b->pitch[i], p->d_vec, p->d_peak, prev);
+                PivParams it = pass_params(p, b->d_fa[i], b->d_fb[i], b->pitch[i], true, p->d_vec,
+                                           p->d_peak, prev);
                 pq.first_task[j] = (int)tasks;
                 pq.first_win[j] = (int)wins;
                 it.flag_base = (int32_t)wins;
@@ -1194,9 +1210,9 @@ int opiv_batch_create(opiv_batch** out, int n_pairs, const uint32_t* widths, con
     for (int i = 0; i < n_pairs && e == cudaSuccess; ++i) {
         const size_t row = (size_t)widths[i] * px_bytes(dtype);
         void *fa = nullptr, *fb = nullptr;
-        if ((e = cudaMalloc(&fa, row * heights[i])) != cudaSuccess) break;
+        if ((e = alloc_frame(&fa, row * heights[i])) != cudaSuccess) break;
         b->d_fa.push_back(fa);
-        if ((e = cudaMalloc(&fb, row * heights[i])) != cudaSuccess) break;
+        if ((e = alloc_frame(&fb, row * heights[i])) != cudaSuccess) break;
         b->d_fb.push_back(fb);
         b->pitch.push_back(row);
     }
@@ -1259,8 +1275,8 @@ int batch_enqueue(opiv_batch* b, cudaStream_t s)
     CUDA_TRY(cudaEventRecord(b->events[ns], s));
     for (int i = 0; i < ns; ++i) CUDA_TRY(cudaStreamWaitEvent(b->streams[i], b->events[ns], 0));
     for (size_t i = 0; i < b->pairs.size(); ++i) {
-        const int rc = opiv_multipass_process_device(b->pairs[i], b->d_fa[i], b->d_fb[i], b->pitch[i],
-                                                     b->streams[i % ns]);
+        const int rc = multipass_device(b->pairs[i], b->d_fa[i], b->d_fb[i], b->pitch[i], true,
+                                        b->streams[i % ns]);
         if (rc != OPIV_OK) return rc;
     }
     for (int i = 0; i < ns; ++i) {
@@ -1571,7 +1587,7 @@ int opiv_batch_process(opiv_batch* b, const void* const* frames_a, const void* c
     for (int i = 0; i < n; ++i) {
         cudaStream_t cs = b->streams[i % ns];
         CUDA_TRY_D(cudaStreamWaitEvent(cs, b->ev_up[i], 0));
-        const int rc = opiv_multipass_process_device(b->pairs[i], b->d_fa[i], b->d_fb[i], b->pitch[i], cs);
+        const int rc = multipass_device(b->pairs[i], b->d_fa[i], b->d_fb[i], b->pitch[i], true, cs);
         if (rc != OPIV_OK) {
             cudaDeviceSynchronize();
             return done(rc);
@@ -1661,7 +1677,7 @@ int opiv_plan_autotune(opiv_plan* plan, const void* d_fa, const void* d_fb, size
         float t_min = 3.4e38f;
         for (int r = 0; r < 4 && rc == OPIV_OK; ++r) {   // one warm-up, three timed
             cudaEventRecord(e0, s);
-            rc = run_pass(plan, d_fa, d_fb, pitch_bytes, plan->d_vec, plan->d_peak, s);
+            rc = run_pass(plan, d_fa, d_fb, pitch_bytes, false, plan->d_vec, plan->d_peak, s);
             cudaEventRecord(e1, s);
             if (rc != OPIV_OK) break;
             const cudaError_t e = cudaEventSynchronize(e1);

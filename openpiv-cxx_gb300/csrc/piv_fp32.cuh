@@ -50,6 +50,7 @@
 #include "offsets.cuh"
 #include "peak_scan.cuh"
 #include "piv_kernels.h"
+#include "row_blocks.h"
 
 namespace opiv {
 namespace fp32 {
@@ -114,15 +115,25 @@ __device__ __forceinline__ void load_row(const PixT* ptr, float2 (&v)[W])
     }
 }
 
+// A row's pixels, one by one, to where its blocks would put them in `line`.
+template <int W, typename PixT>
+__device__ __forceinline__ void row_elements(const PixT* ptr, uint4* line)
+{
+    PixT* to = reinterpret_cast<PixT*>(reinterpret_cast<unsigned char*>(line) + (reinterpret_cast<uintptr_t>(ptr) & 15));
+#pragma unroll 4
+    for (int x = 0; x < W; ++x) to[x] = __ldg(ptr + x);
+}
+
 // A row that starts anywhere (an unaligned grid or pitch, B windows shifted
 // by a previous pass's displacement): the 16-byte blocks covering it are
 // loaded whole and the row is shifted out of them by the start's offset
-// inside its block (a word select, then a byte permute).  The blocks read
-// hold at least one pixel of the row each, so they lie inside the frame's
-// allocation.  (Element by element a 1531 x 1117 u8 pair of 32 px REAL windows
+// inside its block (a word select, then a byte permute).  EDGE: a row whose first
+// or last block would leave the frame (`edge`, row_blocks.h) is put together in
+// `line`, the lane's own shared memory.
+// (Element by element a 1531 x 1117 u8 pair of 32 px REAL windows
 // took 77 us; with everything else as here it takes 41.)
-template <int W, bool B, typename PixT>
-__device__ __forceinline__ void load_row_shifted(const PixT* ptr, float2 (&v)[W])
+template <int W, bool B, bool EDGE, typename PixT>
+__device__ __forceinline__ void load_row_shifted(const PixT* ptr, bool edge, uint4* line, float2 (&v)[W])
 {
     {
         constexpr int NW = W * (int)sizeof(PixT) / 4;   // 32-bit words of the row
@@ -131,14 +142,23 @@ __device__ __forceinline__ void load_row_shifted(const PixT* ptr, float2 (&v)[W]
         const uint4* q = reinterpret_cast<const uint4*>(a & ~(uintptr_t)15);
         const int mis = (int)(a & 15);
         uint32_t w[NW + 4];
+        if (!EDGE || !edge) {
 #pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            const uint4 r = __ldg(q + c);
-            w[4 * c] = r.x; w[4 * c + 1] = r.y; w[4 * c + 2] = r.z; w[4 * c + 3] = r.w;
+            for (int c = 0; c < NC; ++c) {
+                const uint4 r = __ldg(q + c);
+                w[4 * c] = r.x; w[4 * c + 1] = r.y; w[4 * c + 2] = r.z; w[4 * c + 3] = r.w;
+            }
+            uint4 tail = make_uint4(0u, 0u, 0u, 0u);
+            if (mis != 0) tail = __ldg(q + NC);   // only a misaligned row reaches into it
+            w[NW] = tail.x; w[NW + 1] = tail.y; w[NW + 2] = tail.z; w[NW + 3] = tail.w;
+        } else {
+            row_elements<W>(ptr, line);
+#pragma unroll
+            for (int c = 0; c <= NC; ++c) {
+                const uint4 r = line[c];
+                w[4 * c] = r.x; w[4 * c + 1] = r.y; w[4 * c + 2] = r.z; w[4 * c + 3] = r.w;
+            }
         }
-        uint4 tail = make_uint4(0u, 0u, 0u, 0u);
-        if (mis != 0) tail = __ldg(q + NC);   // only a misaligned row reaches into it
-        w[NW] = tail.x; w[NW + 1] = tail.y; w[NW + 2] = tail.z; w[NW + 3] = tail.w;
         const int ws = mis >> 2;
         const uint32_t sel = 0x3210u + 0x1111u * (uint32_t)(mis & 3);
 #pragma unroll
@@ -253,28 +273,41 @@ __device__ __forceinline__ void stage_read(const uint4* tile, int gl, const PixT
 // Both frames' rows of a window (corners ca, cb in their frames): lane = row,
 // registers = columns.  Every lane of the warp calls it; the tile is free
 // again when it returns.
-template <int W, bool AL_A, bool AL_B, typename PixT>
-__device__ __forceinline__ void load_window(const PixT* ca, const PixT* cb, size_t pitch, int gl, uint4* tile,
-                                            float2 (&v)[W])
+template <int W, bool AL_A, bool AL_B, bool EDGE, typename PixT>
+__device__ __forceinline__ void load_window(const PivParams& p, const PixT* ca, const PixT* cb, size_t pitch, int gl,
+                                            uint4* tile, float2 (&v)[W])
 {
     using R = row_stage<W, PixT>;
     const PixT *pa = ca + (size_t)gl * pitch, *pb = cb + (size_t)gl * pitch;   // the lane's rows
+    bool edge_a = false, edge_b = false, edge = false;   // a block of the row leaves the frame; of any of the warp's
+    if constexpr (EDGE) {
+        const size_t extent = frame_extent(p.img_w, p.img_h, p.pitch, sizeof(PixT));
+        edge_a = !AL_A && blocks_leave((uintptr_t)pa, W * sizeof(PixT), (uintptr_t)p.fa, extent);
+        edge_b = !AL_B && blocks_leave((uintptr_t)pb, W * sizeof(PixT), (uintptr_t)p.fb, extent);
+        edge = __any_sync(0xffffffffu, edge_a || edge_b);
+    }
     if constexpr (W == 32 && sizeof(PixT) == 2) {
         static_assert(2 * R::bytes <= (int)sizeof(float2) * W * (W + 1), "both frames' rows fit the tile");
-        uint4 ra[R::NC + 1], rb[R::NC + 1];
-        stage_load<W, AL_A, PixT>(ca, pitch, gl, ra);
-        stage_load<W, AL_B, PixT>(cb, pitch, gl, rb);
-        stage_store<W, AL_A, PixT>(tile, gl, ra);
-        stage_store<W, AL_B, PixT>(tile + R::LD * W, gl, rb);
+        if (!EDGE || !edge) {
+            uint4 ra[R::NC + 1], rb[R::NC + 1];
+            stage_load<W, AL_A, PixT>(ca, pitch, gl, ra);
+            stage_load<W, AL_B, PixT>(cb, pitch, gl, rb);
+            stage_store<W, AL_A, PixT>(tile, gl, ra);
+            stage_store<W, AL_B, PixT>(tile + R::LD * W, gl, rb);
+        } else {
+            row_elements<W>(pa, tile + gl * R::LD);
+            row_elements<W>(pb, tile + (W + gl) * R::LD);
+        }
         __syncwarp();
         stage_read<W, false, AL_A, PixT>(tile, gl, pa, v);
         stage_read<W, true, AL_B, PixT>(tile + R::LD * W, gl, pb, v);
         __syncwarp();
     } else {
         if constexpr (AL_A) load_row<W, false, PixT>(pa, v);
-        else load_row_shifted<W, false, PixT>(pa, v);
+        else load_row_shifted<W, false, EDGE, PixT>(pa, edge_a, tile + gl * R::LD, v);
         if constexpr (AL_B) load_row<W, true, PixT>(pb, v);
-        else load_row_shifted<W, true, PixT>(pb, v);
+        else load_row_shifted<W, true, EDGE, PixT>(pb, edge_b, tile + gl * R::LD, v);
+        if (EDGE && edge) __syncwarp();
     }
     if (sizeof(PixT) <= 2) {
 #pragma unroll
@@ -317,7 +350,9 @@ enum { kStLoad0 = 0, kStCol0 = 1, kStLoad1 = 2, kStCol1 = 3, kStInvA = 4, kStInv
 
 // One task: the 2 * NG windows first = task * 2 * NG ... of pair p, run by
 // the calling warp (its lane groups' shared memory at `dyn_smem`).
-template <int W, int MODE, bool LIMIT, typename PixT, bool PLANES, bool VEC>
+// VEC: every row of frame A, and of B unless displaced, starts on a 16-byte
+// boundary.  EDGE: row blocks may leave a frame.
+template <int W, int MODE, bool LIMIT, typename PixT, bool PLANES, bool VEC, bool EDGE>
 __device__ __forceinline__ void fp32_task(const PivParams& p, const int task, float2* dyn_smem)
 {
     constexpr int NG = 32 / W;          // lane groups per warp
@@ -378,11 +413,11 @@ __device__ __forceinline__ void fp32_task(const PivParams& p, const int task, fl
             } else {
                 uint4* tile = reinterpret_cast<uint4*>(S);
                 if (!VEC)
-                    load_window<W, false, false, PixT>(ca, cb, pitch, gl, tile, v);
+                    load_window<W, false, false, EDGE, PixT>(p, ca, cb, pitch, gl, tile, v);
                 else if (p.prev_disp != nullptr)   // shifted B rows need not be aligned
-                    load_window<W, true, false, PixT>(ca, cb, pitch, gl, tile, v);
+                    load_window<W, true, false, EDGE, PixT>(p, ca, cb, pitch, gl, tile, v);
                 else
-                    load_window<W, true, true, PixT>(ca, cb, pitch, gl, tile, v);
+                    load_window<W, true, true, EDGE, PixT>(p, ca, cb, pitch, gl, tile, v);
             }
             const float2 before = energy;
 #pragma unroll
@@ -652,12 +687,12 @@ extern __shared__ __align__(16) float2 fp32_dyn_smem[];   // rows are staged in 
 template <int W>
 constexpr int min_ctas() { return W == 16 ? 6 : 4; }
 
-template <int W, int MODE, bool LIMIT, typename PixT, bool PLANES, bool VEC>
+template <int W, int MODE, bool LIMIT, typename PixT, bool PLANES, bool VEC, bool EDGE>
 __global__ void __launch_bounds__(32 * kWarps, min_ctas<W>())
 piv_fp32_kernel(const PivParams p)
 {
     after_previous();
-    fp32_task<W, MODE, LIMIT, PixT, PLANES, VEC>(p, (int)blockIdx.x * kWarps + (int)(threadIdx.x >> 5),
+    fp32_task<W, MODE, LIMIT, PixT, PLANES, VEC, EDGE>(p, (int)blockIdx.x * kWarps + (int)(threadIdx.x >> 5),
                                                  fp32_dyn_smem);
 }
 
@@ -706,10 +741,24 @@ piv_fp32_queue_kernel(const __grid_constant__ PivQueue q)
         for (int t = (int)t0 + warp; t < t1; t += kWarps) {
             const int j = __ldg(q.task_item + t);
             const PivParams& p = warp_item(q, j, my_item);
-            fp32_task<W, MODE, LIMIT, PixT, false, VEC>(p, t - q.first_task[j], fp32_dyn_smem);
+            fp32_task<W, MODE, LIMIT, PixT, false, VEC, false>(p, t - q.first_task[j], fp32_dyn_smem);
             __syncwarp();   // the descriptor is overwritten by the next task
         }
     }
+}
+
+// Whether a block of a pass's rows may leave one of its frames; displaced
+// windows of frame B can lie anywhere in it.
+inline bool blocks_may_leave(const PivParams& p, int w, size_t px)
+{
+    for (const void* f : { p.fa, p.fb }) {
+        const uintptr_t lo = (uintptr_t)f;
+        if (p.prev_disp != nullptr && (lo % 16 != 0 || (lo + frame_extent(p.img_w, p.img_h, p.pitch, px)) % 16 != 0))
+            return true;
+        if (grid_blocks_leave(lo, p.img_w, p.img_h, p.pitch, px, w, p.gx0, p.gy0, p.gdx, p.gdy, p.gnx, p.n_win / p.gnx))
+            return true;
+    }
+    return false;
 }
 
 template <int W, int MODE, bool LIMIT, typename PixT, bool PLANES>
@@ -724,19 +773,26 @@ cudaError_t launch_t(const PivParams& p, cudaStream_t s)
                      ((uintptr_t)p.fb % 16 == 0) && (p.pitch % 16 == 0) &&
                      (((size_t)p.gx0 * px) % 16 == 0) && (((size_t)p.gdx * px) % 16 == 0) &&
                      ((W * px) % 16 == 0);
+    // rows read as blocks where one would leave a frame: looking for them costs
+    // every window 2 % (4096 x 4096, 32 px at step 8: 733 us, 716 without), so only
+    // passes that may meet one do
+    const bool edge = !PLANES && !p.frames_padded && (!vec || p.prev_disp != nullptr) && blocks_may_leave(p, W, px);
     const size_t smem = sizeof(float2) * kWarps * NG * group_smem_float2<W>();
-    auto kern = vec ? piv_fp32_kernel<W, MODE, LIMIT, PixT, PLANES, true>
-                    : piv_fp32_kernel<W, MODE, LIMIT, PixT, PLANES, false>;
+    auto kern = vec ? piv_fp32_kernel<W, MODE, LIMIT, PixT, PLANES, true, false>
+                    : piv_fp32_kernel<W, MODE, LIMIT, PixT, PLANES, false, false>;
+    if constexpr (!PLANES)
+        if (edge) kern = piv_fp32_kernel<W, MODE, LIMIT, PixT, PLANES, false, true>;
     // per instantiation, load path and device
-    static std::atomic<uint64_t> attr_done[2] = { { 0 }, { 0 } };
+    static std::atomic<uint64_t> attr_done[3] = { { 0 }, { 0 }, { 0 } };
+    const int path = edge ? 2 : vec;
     int dev = 0;
     cudaGetDevice(&dev);
     const uint64_t bit = 1ull << (dev & 63);
-    if (!(attr_done[vec].load() & bit)) {
+    if (!(attr_done[path].load() & bit)) {
         const cudaError_t e =
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        attr_done[vec].fetch_or(bit);
+        attr_done[path].fetch_or(bit);
     }
     return launch_dependent(kern, (unsigned)blocks, 32 * kWarps, smem, s, p);
 }
@@ -780,7 +836,7 @@ piv_fp32_list_kernel(const __grid_constant__ PivQueue q)
     if (t >= q.first_task[q.n_items]) return;   // warp-uniform
     const int j = __ldg(q.task_item + t);
     const PivParams& p = warp_item(q, j, reinterpret_cast<PivParams*>(s_items) + warp);
-    fp32_task<W, MODE, LIMIT, PixT, false, VEC>(p, t - q.first_task[j], fp32_dyn_smem);
+    fp32_task<W, MODE, LIMIT, PixT, false, VEC, false>(p, t - q.first_task[j], fp32_dyn_smem);
 }
 
 // ---- the persistent queue form ------------------------------------------------

@@ -46,6 +46,7 @@ struct alignas(16) PivParams {
     // (a queue's is one counter, reset by its launcher).
     unsigned int* flag_count = nullptr;
     int32_t* flag_list = nullptr;
+    int32_t frames_padded = 0;         // whole 16-byte blocks of the frames may be read (the library's own)
     int32_t flag_base = 0;             // added to a flagged window's index (a queue's list)
     // the flagged windows' records, by their place in the list.  A pass that
     // flags more windows than flag_cap takes the FP64 transforms for all of
