@@ -192,7 +192,7 @@ struct opiv_plan {
     flag_record* d_flag_recs = nullptr; // a record for every window (none in tensor-core-only plans)
     int32_t flag_cap = 0;
     double2* d_tw = nullptr;            // forward then reverse, ia entries each
-    bool flags = false;                 // the last pass was an FP32 one: d_flag_count[2] is its count
+    bool flags = false;                 // the last pass was an FP32 one: its counts are in d_flag_count
     bool timing = false;
     cudaEvent_t ev[3] = { nullptr, nullptr, nullptr };   // fp32 start, fp32 end, exact end
     int32_t* d_disp = nullptr;          // integer displacements (multi-pass plans)
@@ -732,26 +732,43 @@ int opiv_process_pairs(opiv_plan* plan, int64_t n_pairs, const void* const* fram
 
 namespace {
 
-// Counter `at` of the plan's last pass.
-int64_t last_flag_counter(opiv_plan* plan, int at)
+// The counters of the plan's last pass into `words`; false (and zeros) after
+// a pass of a precision that flags nothing, or an error (in *rc).
+bool last_flag_counters(opiv_plan* plan, unsigned int* words, int* rc)
 {
-    if (!plan) return fail(OPIV_ERR_ARG, "plan is null");
-    unsigned int count = 0;
-    if (!plan->flags) return 0;   // the other precisions flag nothing
+    std::fill(words, words + kFlagCounters, 0u);
+    *rc = plan ? OPIV_OK : fail(OPIV_ERR_ARG, "plan is null");
+    if (!plan || !plan->flags) return false;
     int prev = 0;
     cudaGetDevice(&prev);
     cudaSetDevice(plan->device);
     cudaDeviceSynchronize();
-    const cudaError_t e = cudaMemcpy(&count, plan->d_flag_count + at, sizeof count, cudaMemcpyDeviceToHost);
+    const cudaError_t e =
+        cudaMemcpy(words, plan->d_flag_count, kFlagCounters * sizeof(unsigned int), cudaMemcpyDeviceToHost);
     cudaSetDevice(prev);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpy(flag count)");
-    return (int64_t)count;
+    if (e != cudaSuccess) *rc = cuda_fail(e, "cudaMemcpy(flag counters)");
+    return e == cudaSuccess;
 }
 
 }  // namespace
 
-int64_t opiv_plan_exact_count(opiv_plan* plan) { return last_flag_counter(plan, 2); }
-int64_t opiv_plan_settled_count(opiv_plan* plan) { return last_flag_counter(plan, 4); }
+int64_t opiv_plan_exact_count(opiv_plan* plan)
+{
+    unsigned int words[kFlagCounters];
+    int rc;
+    return last_flag_counters(plan, words, &rc) ? (int64_t)words[kLastFlagged] : (int64_t)rc;
+}
+
+int64_t opiv_plan_settled_count(opiv_plan* plan)
+{
+    unsigned int words[kFlagCounters];
+    int rc;
+    if (!last_flag_counters(plan, words, &rc)) return rc;
+    uint64_t before, after;
+    std::memcpy(&before, words + kSettledBefore, sizeof before);
+    std::memcpy(&after, words + kSettled, sizeof after);
+    return (int64_t)(after - before);
+}
 
 int opiv_multipass_create(opiv_multipass** out, uint32_t img_w, uint32_t img_h, int dtype,
                           int n_passes, const uint32_t* ia, const uint32_t* step, int mode,

@@ -508,10 +508,12 @@ piv_exact_kernel(const PivParams p, int W, int mode, int limit)
     __shared__ int row_count[kMaxW];
     __shared__ int total_cand;
     if (LIST) after_previous();
-    const int64_t nwork = LIST ? (int64_t)min(*p.flag_count, (unsigned int)p.flag_room) : p.n_win;
+    const int64_t nwork = LIST ? (int64_t)min(p.flag_count[kFlagged], (unsigned int)p.flag_room) : p.n_win;
     int sy0, sy1, sx0, sx1;
     scan_range(W, limit, sy0, sy1, sx0, sx1);
     unsigned int settled = 0;
+    unsigned long long* words = LIST ? reinterpret_cast<unsigned long long*>(p.flag_count) : nullptr;
+    const unsigned long long settled_before = LIST ? words[kSettled / 2] : 0;
     for (int64_t item = blockIdx.x; item < nwork; item += gridDim.x) {
         const int64_t w = LIST ? (int64_t)p.flag_list[item] : item;
         if constexpr (LIST) {
@@ -529,15 +531,15 @@ piv_exact_kernel(const PivParams p, int W, int mode, int limit)
         // them (every CTA has read the count by then), so that a pass is two
         // launches: a memset before them and a copy of the count after them
         // were half of a small pass's time (160 x 128 px: 25.8 -> 14.3 us)
-        if (threadIdx.x == 0 && settled > 0) {
-            atomicAdd(p.flag_count + 3, settled);
-            __threadfence();   // before this CTA counts as done
-        }
-        if (threadIdx.x == 0 && atomicAdd(p.flag_count + 1, 1u) == gridDim.x - 1) {
-            p.flag_count[2] = (unsigned int)nwork;
-            p.flag_count[4] = nwork > 0 ? atomicExch(p.flag_count + 3, 0u) : 0u;   // (a round trip to memory)
-            p.flag_count[1] = 0u;
-            p.flag_count[0] = 0u;
+        if (threadIdx.x == 0) {
+            const uint64_t before = atomicAdd(words + kDone / 2, done_add(settled));
+            if (last_done(before, gridDim.x)) {
+                atomicAdd(words + kDone / 2, 0ull - gridDim.x);
+                p.flag_count[kLastFlagged] = (unsigned int)nwork;
+                words[kSettledBefore / 2] = settled_before;
+                words[kSettled / 2] = all_settled(before, settled);
+                p.flag_count[kFlagged] = 0u;
+            }
         }
     }
 }

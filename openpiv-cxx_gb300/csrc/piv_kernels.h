@@ -3,6 +3,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "flag_counters.h"
 #include "openpiv_gb300.h"
 
 namespace opiv {
@@ -41,9 +42,9 @@ struct alignas(16) PivParams {
     opiv_vector* out_vec = nullptr;
     int32_t* out_peak = nullptr;       // may be null
     // windows whose FP32 decisions are not certain (see piv_fp32.cu).  The
-    // single-pair passes' flag_count is kFlagCounters counters, zero before a
-    // pass: windows flagged, and the exact launch's, which leaves them zero
-    // (a queue's is one counter, reset by its launcher).
+    // single-pair passes' flag_count is kFlagCounters words, zero before a
+    // pass, and the exact launch leaves them so (flag_counters.h; a queue's is
+    // one counter, reset by its launcher).
     unsigned int* flag_count = nullptr;
     int32_t* flag_list = nullptr;
     int32_t frames_padded = 0;         // whole 16-byte blocks of the frames may be read (the library's own)
@@ -74,11 +75,6 @@ struct alignas(16) PivParams {
     int32_t* out_disp = nullptr;       // this pass's integer displacements (may be null)
     int* status = nullptr;             // tensor-core kernel: set to 1 if an MMA wait gave up
 };
-
-// flag_count[0]: windows flagged so far; [1]: CTAs of the exact launch that
-// are done; [2]: windows flagged in the last pass; [3]: flagged windows decided
-// from exact sums so far; [4]: in the last pass.
-constexpr int kFlagCounters = 5;
 
 // Programmatic dependent launch of a pass's kernels on one stream: the launch
 // is prepared while the kernel before it still runs, and the kernel calls
