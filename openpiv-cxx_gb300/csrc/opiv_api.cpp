@@ -370,14 +370,17 @@ int run_pass(opiv_plan* p, const void* fa, const void* fb, size_t pitch, bool pa
     if (p->timing) CUDA_TRY(cudaEventRecord(p->ev[0], s));
     CUDA_TRY(launch_piv_fp32(k, (int)p->ia, p->dtype, p->mode, p->limit, false, s));
     ++g_launches;
-    if (p->timing) CUDA_TRY(cudaEventRecord(p->ev[1], s));
+    // no return between the launches: the second leaves the counters of the
+    // first's flagged windows as the next pass wants them
+    const cudaError_t between = p->timing ? cudaEventRecord(p->ev[1], s) : cudaSuccess;
     const cudaError_t e =
         launch_piv_exact(k, (int)p->ia, p->dtype, p->mode, p->limit, true, exact_blocks(p->device), s);
-    if (e != cudaSuccess) {   // the counters as the next pass wants them
+    if (e != cudaSuccess) {
         cudaMemsetAsync(k.flag_count, 0, kFlagCounters * sizeof(unsigned int), s);
         return cuda_fail(e, "launch_piv_exact");
     }
     ++g_launches;
+    CUDA_TRY(between);
     if (p->timing) CUDA_TRY(cudaEventRecord(p->ev[2], s));
     return OPIV_OK;
 }
