@@ -699,9 +699,10 @@ piv_tc48_kernel(const PivParams p, const uint4* __restrict__ consts)
 
         // ---- find_peaks: thread = (column x < 48 of 64, 24-row block); the
         // block's candidate rows roll through registers, neighbouring columns
-        // come from the plane (shuffles, with the edge lanes' own loads, took
-        // five shared-memory cycles a row where this takes three); branch-free
-        // top two
+        // come from the plane: three shared-memory cycles a row for the second
+        // warp of a block, six for the first, whose loads each meet one bank twice
+        // (the shift of the second half); shuffles and the edge lanes' own loads took
+        // five for either; branch-free top two
         {
             const int xs = tid & 63, yb = (tid >> 6) * 24;
             const bool col_ok = xs >= SX0 && xs < SX1;

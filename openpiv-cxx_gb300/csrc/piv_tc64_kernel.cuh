@@ -552,8 +552,9 @@ piv_tc64_kernel(const PivParams p, const uint4* __restrict__ consts)
 
         // ---- find_peaks: thread = (column x, 32-row block); the block's
         // candidate rows roll through registers, neighbouring columns come
-        // from the plane (shuffles, with the edge lanes' own loads, took five
-        // shared-memory cycles a row where this takes three); branch-free top two
+        // from the plane: five shared-memory cycles a row, as many as shuffles and
+        // the edge lanes' own loads took (the shift of the second half makes the left
+        // and the right load of every warp meet one bank twice); branch-free top two
         {
             const int xs = tid & 63, yb = (tid >> 6) * 32;
             const bool col_ok = xs >= SX0 && xs < SX1;

@@ -59,3 +59,30 @@ def test_same_result_whatever_the_order(ia, step, h, w):
             v, k, _ = batch.results(0, 0)
             assert np.array_equal(v, vec, equal_nan=True) and np.array_equal(k, pk), schedule
     batch.close()
+
+
+def test_more_flagged_windows_than_records():
+    """The allocation-free call on a grid whose flag list leaves its fixed
+    scratch fewer records than windows are flagged: the FP64 transforms decide
+    all of them, as they do for a plan of that precision."""
+    torch = pytest.importorskip("torch")
+    ia, step, h, w = 16, 2, 1024, 1024
+    pair = flat_frames(h, w, 60000, SPREAD[ia], 5)
+    plan = og.Plan(w, h, np.uint16, ia, step)
+    plan.process(*pair)
+    # 4 MiB of scratch, 4 bytes of list a window, 40 bytes a record
+    assert plan.exact_count() > ((4 << 20) - 4 * plan.n) // 40, "the frames no longer flag enough windows"
+    plan.set_precision(og.PREC_FP64)
+    vec, pk = plan.process(*pair)
+    d = [torch.from_numpy(f.view(np.int16)).cuda() for f in pair]
+    out = torch.zeros((plan.n, 5), dtype=torch.float32, device="cuda")
+    codes = torch.zeros(plan.n, dtype=torch.int32, device="cuda")
+    og.process_pair_device_noalloc(d[0].data_ptr(), d[1].data_ptr(), 2 * w, w, h, np.uint16, ia, step, step,
+                                   og.CORR_COMPLEX, False, out.data_ptr(), codes.data_ptr())
+    torch.cuda.synchronize()
+    got, code = out.cpu().numpy(), codes.cpu().numpy()
+    exact = (code >= 0) & ((code & og.PEAK_EXACT) != 0)
+    assert exact.sum() > plan.n // 2
+    assert np.array_equal(code[exact] & og.PEAK_MASK, pk[exact] & og.PEAK_MASK)
+    assert np.array_equal(got[exact], vec[exact], equal_nan=True)
+    plan.close()
