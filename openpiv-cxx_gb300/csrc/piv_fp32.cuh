@@ -115,13 +115,16 @@ __device__ __forceinline__ void load_row(const PixT* ptr, float2 (&v)[W])
     }
 }
 
-// A row's pixels, one by one, to where its blocks would put them in `line`.
+// A row, byte by byte, to where its blocks would put it in `line` (32 loads in
+// flight: passes whose grid ends at the frame's corners take up to 1 us longer
+// for these rows, 1.3 with 8).
 template <int W, typename PixT>
-__device__ __forceinline__ void row_elements(const PixT* ptr, uint4* line)
+__device__ __forceinline__ void row_bytes(const PixT* ptr, uint4* line)
 {
-    PixT* to = reinterpret_cast<PixT*>(reinterpret_cast<unsigned char*>(line) + (reinterpret_cast<uintptr_t>(ptr) & 15));
-#pragma unroll 4
-    for (int x = 0; x < W; ++x) to[x] = __ldg(ptr + x);
+    const unsigned char* from = reinterpret_cast<const unsigned char*>(ptr);
+    unsigned char* to = reinterpret_cast<unsigned char*>(line) + (reinterpret_cast<uintptr_t>(ptr) & 15);
+#pragma unroll 32
+    for (int i = 0; i < W * (int)sizeof(PixT); ++i) to[i] = __ldg(from + i);
 }
 
 // A row that starts anywhere (an unaligned grid or pitch, B windows shifted
@@ -152,7 +155,7 @@ __device__ __forceinline__ void load_row_shifted(const PixT* ptr, bool edge, uin
             if (mis != 0) tail = __ldg(q + NC);   // only a misaligned row reaches into it
             w[NW] = tail.x; w[NW + 1] = tail.y; w[NW + 2] = tail.z; w[NW + 3] = tail.w;
         } else {
-            row_elements<W>(ptr, line);
+            row_bytes<W>(ptr, line);
 #pragma unroll
             for (int c = 0; c <= NC; ++c) {
                 const uint4 r = line[c];
@@ -295,8 +298,8 @@ __device__ __forceinline__ void load_window(const PivParams& p, const PixT* ca, 
             stage_store<W, AL_A, PixT>(tile, gl, ra);
             stage_store<W, AL_B, PixT>(tile + R::LD * W, gl, rb);
         } else {
-            row_elements<W>(pa, tile + gl * R::LD);
-            row_elements<W>(pb, tile + (W + gl) * R::LD);
+            row_bytes<W>(pa, tile + gl * R::LD);
+            row_bytes<W>(pb, tile + (W + gl) * R::LD);
         }
         __syncwarp();
         stage_read<W, false, AL_A, PixT>(tile, gl, pa, v);

@@ -1,5 +1,5 @@
 """Frames whose first and last pixels are a window's: rows whose 16-byte blocks
-would leave the frame are read pixel by pixel, at every kind of offset from a
+would leave the frame are read byte by byte, at every kind of offset from a
 block boundary and with odd pitches, and give what the packed, aligned frames
 give (the arithmetic is the same whatever the alignment).
 """
