@@ -72,8 +72,9 @@ L2_ROTATION = 4
 KERNEL_TRAFFIC = {
     "tc": {"bytes": 67_309_056 + 95_744,
            "sources": {"piv_tc_kernel.cuh": "e89e8fd5118876f1", "tc_ptx.cuh": "74cf252d23d6309a"}},
-    "fp32": {"bytes": 67_160_576 + 4_210_176,
-             "sources": {"piv_fp32.cuh": "bf57c59dd05ec6c9", "fft_reg.cuh": "59d479598caf2c38"}},
+    "fp32": {"bytes": 67_164_160 + 3_619_328,
+             "sources": {"piv_fp32.cuh": "4f8e521dbedb6336", "fft_reg.cuh": "4a8d42e5baf7a0fd",
+                         "peak_scan.cuh": "50d2f2916b9962ca"}},
 }
 
 

@@ -25,7 +25,7 @@
 // A 2048 x 2048 float pair, 32 px windows at step 16 (16,129 windows), both
 // outputs: 157 -> 50 us.  Re-reading the five taps of both frames for every
 // pixel took sixteen loads a pixel where this takes two.  Bound by issue
-// slots (66 % busy at 16 warps an SM: about 2,300 instructions a window, of
+// slots (65 % busy at 16 warps an SM: about 2,300 instructions a window, of
 // them 640 FMAs, 192 shuffles, 64 loads and 64 gradient updates, and their
 // addresses); 128 registers hold a 32 px window's two frames.
 //

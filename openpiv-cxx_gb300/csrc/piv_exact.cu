@@ -294,11 +294,12 @@ __device__ __forceinline__ void exact_window(const PivParams& p, const int64_t w
 // the totals of the plain and the weighted sums: whole numbers again.
 // Returns false, with nothing written, where the exact kernel has to decide:
 // ties and signs within the reference's own FP64 rounding, more than
-// kMaxCand candidates, non-finite planes.
+// kMaxCand candidates, windows with infinite or huge pixels.
 // The launch's time with the FP64 transforms and with this: a 4096 x 4096
 // pass of 32 px windows at step 8 (4 flagged) 111 -> 12 us; 2048 x 1536, 16 px
 // at step 8 (78 flagged) 48 -> 9 us; 2048 x 2048, 64 px at step 16 (2 flagged)
-// 360 -> 20 us; none flagged 3 us.  What is left is a chain of dependent loads,
+// 360 -> 19 us; 15,625 of 15,625 32 px windows flagged 7125 -> 349 us (with room for
+// the records of one in 32 before); none flagged 3 us.  What is left is a chain of dependent loads,
 // block barriers and FP64 logarithms of one window.
 struct refine_shared {
     long long val[5 * kMaxCand];   // or doubles: centre, left, right, up, down
